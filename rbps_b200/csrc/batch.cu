@@ -382,7 +382,6 @@ struct rbps_batch
     uint32_t gjk_cap = 0, gjk_slots = 0;
     PhaseLaunch phase{};      // grid / block of each phase kernel
     FlatLaunch flat{};        // flat colored pipeline
-    bool use_flat = false;
     uint32_t *wcoff = nullptr, *gcol = nullptr, *sbodies = nullptr, *sjoints = nullptr, *sjcoff = nullptr;
     uint2 *nlist = nullptr;
     uint4 *nglob = nullptr; // global collider / body indices beside nlist
@@ -487,13 +486,9 @@ struct rbps_batch
         if (flat.side)
         {
             cudaStreamSynchronize(flat.side);
-            for (int k = 0; k < 8; ++k)
-            {
-                if (flat.fork[k])
-                    cudaEventDestroy(flat.fork[k]);
-                if (flat.join[k])
-                    cudaEventDestroy(flat.join[k]);
-            }
+            for (cudaEvent_t e : {flat.fork, flat.join})
+                if (e)
+                    cudaEventDestroy(e);
             cudaStreamDestroy(flat.side);
         }
         if (graph_exec)
@@ -927,6 +922,7 @@ namespace
     constexpr int kMaxBlockHost = 256; // block of the flat kernels (their __launch_bounds__)
     constexpr uint32_t kBlockTeamBodies = 256; // colored batches: worlds this large step on a whole CTA
     constexpr uint32_t kPairTeamBodies = 96;   // ... and worlds this large on half a CTA
+    constexpr size_t kSmemWorldsMax = 226 * 1024; // bytes of world copies a CTA can open (227 KB less the scan words)
     constexpr uint32_t kSmemBodiesMax = 1024;   // bodies a CTA world keeps in shared memory (137 KB in FP32)
 } // namespace
 
@@ -950,12 +946,16 @@ static int set_team_split(rbps_batch *b, uint32_t threshold, uint32_t pair)
     b->n_block_worlds = nbw;
     b->n_pair_worlds = npw;
     b->flat.grid_solve = (int)(nbw + (npw + 1) / 2 + (ns - nbw - npw + 3) / 4);
-    auto round16 = [](uint32_t x) { return (x + 15u) / 16u * 16u; };
-    b->smem_cap_warp = round16(pair);
-    b->smem_cap_pair = npw ? round16(std::min<uint32_t>(b->wdev[b->small_ids[nbw]].n_bodies, kSmemBodiesMax)) : 0;
-    b->smem_cap_block = 0;
-    if (nbw)
-        b->smem_cap_block = round16(std::min<uint32_t>(b->wdev[b->small_ids[0]].n_bodies, kSmemBodiesMax));
+    // bodies of each of a CTA's `copies` worlds, as many as fit its shared memory
+    auto cap = [](uint32_t n, uint32_t copies) {
+        uint32_t c = (std::min(n, kSmemBodiesMax) + 15u) / 16u * 16u;
+        while (c && copies * smem_world_bytes<T, P>(c) > kSmemWorldsMax)
+            c -= 16u;
+        return c;
+    };
+    b->smem_cap_warp = cap(pair, 4);
+    b->smem_cap_pair = npw ? cap(b->wdev[b->small_ids[nbw]].n_bodies, 2) : 0;
+    b->smem_cap_block = nbw ? cap(b->wdev[b->small_ids[0]].n_bodies, 1) : 0;
     b->flat.substep_smem = std::max({4 * smem_world_bytes<T, P>(b->smem_cap_warp),
                                      2 * smem_world_bytes<T, P>(b->smem_cap_pair),
                                      smem_world_bytes<T, P>(b->smem_cap_block)});
@@ -1015,7 +1015,9 @@ static int commit_typed(rbps_batch *b)
         for (const auto &j : hw.joints)
             rows += j.type == RBPS_JOINT_REVOLUTE ? 4 : (j.type == RBPS_JOINT_PRISMATIC ? 3 : 2); // fixed, spherical: 2
         d.n_rows = rows;
-        // greedy joint colouring by shared dynamic bodies
+        // joints by shared dynamic bodies: greedy colours, or in reference
+        // order levels (one more than the highest earlier joint's on either
+        // body), which relax in parallel with the bits of the list order
         {
             std::vector<uint32_t> color(d.n_joints, 0);
             uint32_t ncol = 0;
@@ -1028,8 +1030,11 @@ static int commit_typed(rbps_batch *b)
                     if (hw.bodies[bb].type != RBPS_BODY_STATIC)
                         used.insert(used.end(), body_cols[bb].begin(), body_cols[bb].end());
                 uint32_t c = 0;
-                while (std::find(used.begin(), used.end(), c) != used.end())
-                    ++c;
+                if (b->desc.solve_mode == RBPS_SOLVE_REFERENCE_ORDER)
+                    c = used.empty() ? 0u : *std::max_element(used.begin(), used.end()) + 1u;
+                else
+                    while (std::find(used.begin(), used.end(), c) != used.end())
+                        ++c;
                 color[j] = c;
                 ncol = std::max(ncol, c + 1);
                 for (uint32_t bb : {jd.body_1, jd.body_2})
@@ -1475,9 +1480,9 @@ static int commit_typed(rbps_batch *b)
             return fail(RBPS_ERR_CUDA, "cooperative step kernel cannot be resident");
         b->grid_big = per_sm * b->sm_count;
     }
-    b->n_counters = 2 + 4 * (uint32_t)b->desc.substeps;
-    // ---- flat colored pipeline over the small worlds
-    if (!b->small_ids.empty() && b->desc.solve_mode == RBPS_SOLVE_COLORED)
+    b->n_counters = 2; // the frame's and the stats phase's
+    // ---- flat pipeline over the small worlds
+    if (!b->small_ids.empty())
     {
         const uint32_t ns = (uint32_t)b->small_ids.size();
         size_t cand_cap = 0;
@@ -1530,14 +1535,10 @@ static int commit_typed(rbps_batch *b)
         b->flat.block_solve = 128;
         if ((rc = set_team_split<T, P>(b, kBlockTeamBodies, kPairTeamBodies)))
             return rc;
-        b->use_flat = true;
         // side stream + events for the parallel narrowphase kernels
         CU(cudaStreamCreateWithFlags(&b->flat.side, cudaStreamNonBlocking));
-        for (int k = 0; k < 8; ++k)
-        {
-            CU(cudaEventCreateWithFlags(&b->flat.fork[k], cudaEventDisableTiming));
-            CU(cudaEventCreateWithFlags(&b->flat.join[k], cudaEventDisableTiming));
-        }
+        CU(cudaEventCreateWithFlags(&b->flat.fork, cudaEventDisableTiming));
+        CU(cudaEventCreateWithFlags(&b->flat.join, cudaEventDisableTiming));
     }
     // ---- GJK pass: only batches with hull colliders reach it
     {
@@ -1643,22 +1644,15 @@ static long enqueue_step(rbps_batch *b, const Engine<T, P> &e)
     {
         if (cudaMemsetAsync(b->work_counter, 0, 4 * (size_t)b->n_counters, b->stream) != cudaSuccess)
             return RBPS_ERR_CUDA;
-        if (b->use_flat)
-        {
-            if (launch_step_flat<T, P>(e, b->phase, b->flat, b->stream) != cudaSuccess)
-                return RBPS_ERR_CUDA;
-            // frame, prefix, 3 class-sort kernels, stats (only with dumps:
-            // otherwise the last substep writes them); per substep the three
-            // narrowphase kernels, the GJK pass (batches with hulls) and the
-            // substep
-            launches += (e.dump_cc || b->desc.substeps < 1 ? 6 : 5) + (long)b->desc.substeps * (e.gjk_list ? 5 : 4);
-        }
-        else
-        {
-            if (launch_step_phases<T, P>(e, b->phase, b->stream) != cudaSuccess)
-                return RBPS_ERR_CUDA;
-            launches += b->n_counters + (e.gjk_list ? (long)b->desc.substeps : 0); // + the GJK passes
-        }
+        if (launch_step_flat<T, P>(e, b->phase, b->flat, b->stream) != cudaSuccess)
+            return RBPS_ERR_CUDA;
+        // frame, prefix, 3 class-sort kernels, stats (only with dumps:
+        // otherwise the last substep writes them); per substep the three
+        // narrowphase kernels, the GJK pass (batches with hulls) and the
+        // substep (three kernels in float reference order)
+        const long solve = e.solve_mode != 1 && sizeof(T) == 4 ? 3 : 1;
+        launches += (e.dump_cc || b->desc.substeps < 1 ? 6 : 5) +
+                    (long)b->desc.substeps * (3 + solve + (e.gjk_list ? 1 : 0));
     }
     for (uint32_t w : b->big_ids)
     {
@@ -2528,7 +2522,7 @@ static int apply_launch(rbps_batch *b, int frame_block, int narrow_grid)
         b->phase.block[kKFrame] = frame_block;
         b->phase.grid[kKFrame] = std::min<int>((int)b->small_ids.size(), per_sm * b->sm_count);
     }
-    if (b->use_flat)
+    if (!b->small_ids.empty())
         b->flat.grid_narrow = std::max(1, narrow_grid);
     b->graph_key = -1; // recapture the step graph with the new shapes
     return RBPS_OK;
@@ -2582,7 +2576,7 @@ static int autotune_typed(rbps_batch *b, int trials, rbps_tune_result *out)
     const uint32_t tb0 = b->team_bodies, pb0 = b->pair_bodies;
     uint32_t best_t = tb0, best_p = pb0;
     uint32_t n_trials = (uint32_t)cand.size();
-    if (!rc && b->use_flat)
+    if (!rc && !b->small_ids.empty())
     {
         rc = apply_launch<T, P>(b, best_c.first, best_c.second);
         const std::pair<uint32_t, uint32_t> splits[] = {{128u, 128u}, {96u, 96u}, {192u, 64u}, {256u, 64u},
@@ -2638,7 +2632,7 @@ static int autotune_typed(rbps_batch *b, int trials, rbps_tune_result *out)
         *ms_out = ms / trials;
         return RBPS_OK;
     };
-    if (!rc && b->use_flat)
+    if (!rc && !b->small_ids.empty())
     {
         for (uint32_t npw : {64u, 128u, 256u})
         {
@@ -2708,7 +2702,7 @@ template <class T, class P>
 static int set_launch_typed(rbps_batch *b, const rbps_tune_result *cfg)
 {
     int rc;
-    if (b->use_flat && (cfg->team_bodies || cfg->pair_bodies) &&
+    if (!b->small_ids.empty() && (cfg->team_bodies || cfg->pair_bodies) &&
         (rc = set_team_split<T, P>(b, cfg->team_bodies ? cfg->team_bodies : b->team_bodies,
                                    cfg->pair_bodies ? cfg->pair_bodies : b->pair_bodies)))
         return rc;

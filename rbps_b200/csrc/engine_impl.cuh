@@ -72,7 +72,8 @@ namespace rbps_gpu
         CandContacts<T, P> *cc;
         uint32_t *color;
         unsigned long long *bmask, *bprio, *claim;
-        uint32_t *corder, *misc, *act, *alist;
+        uint32_t *corder, *misc, *act, *alist, *loff;
+        uint2 *lrec;
         float4 *yz;
     };
 
@@ -103,6 +104,8 @@ namespace rbps_gpu
         s.misc = (uint32_t *)(base + L.misc);
         s.act = (uint32_t *)(base + L.act);
         s.alist = (uint32_t *)(base + L.alist);
+        s.lrec = (uint2 *)(base + L.lrec);
+        s.loff = (uint32_t *)(base + L.loff);
         return s;
     }
 
@@ -812,26 +815,178 @@ namespace rbps_gpu
         return n_sap + W.n_pc;
     }
 
+    // Asks L2 for every 128-byte line of [p, p + bytes) (prefetch.global.L2).
+    __device__ __forceinline__ void prefetch_l2_range(const void *p, size_t bytes)
+    {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+        for (uintptr_t l = a & ~uintptr_t(127); l < a + bytes; l += 128)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(l));
+    }
+
+    // The contacting candidates of a grid world into S.alist, in candidate
+    // order, their colours reset; the others marked idle.  Returns the count.
+    template <class T, class P>
+    __device__ uint32_t compact_grid(const GridTeam &tm, const Scr<T, P> &S, uint32_t n_cand, BlockShared &sh)
+    {
+        for (uint32_t c = tm.rank(); c < n_cand; c += tm.size())
+            S.act[c] = S.cc[c].n > 0 ? 1u : 0u;
+        tm.sync();
+        const uint32_t n_act = team_excl_scan(tm, S.act, S.act, n_cand, S.tile_sums, sh);
+        for (uint32_t c = tm.rank(); c < n_cand; c += tm.size())
+        {
+            if (S.cc[c].n > 0)
+                S.alist[S.act[c]] = c;
+            S.color[c] = S.cc[c].n > 0 ? 0xffffffffu : kColorIdle;
+        }
+        tm.sync();
+        return n_act;
+    }
+
+    // Level of every active candidate q in [0, n) of S.lrec into lvl, on one
+    // warp: one more than the highest level of the earlier candidates on its
+    // dynamic bodies.  last[b] (zeroed) is the first level free on body b.
+    // Candidates are taken 32 at a time; within the 32, lane j's level is
+    // final once the lanes before it have been passed round, so one loop of
+    // 32 shuffles settles them, and the last lane on a body writes its word.
+    // Returns the number of levels.
+    __device__ __forceinline__ uint32_t levels_warp(const uint2 *lrec, uint32_t n, uint32_t *last, uint32_t *lvl)
+    {
+        const uint32_t lane = lane_id();
+        uint32_t top = 0;
+        uint2 ahead = lane < n ? lrec[lane] : make_uint2(0u, 0u);
+        for (uint32_t k0 = 0; k0 < n; k0 += 32)
+        {
+            const uint2 r = ahead;
+            const uint32_t kn = k0 + 32 + lane;
+            ahead = kn < n ? lrec[kn] : make_uint2(0u, 0u);
+            // a record without its top bit is a static body: nothing waits on it
+            const bool da = r.x >> 31, db = r.y >> 31;
+            const uint32_t a = r.x & 0x7fffffffu, b = r.y & 0x7fffffffu;
+            uint32_t l = max(da ? last[a] : 0u, db ? last[b] : 0u);
+            bool last_a = da, last_b = db; // no later lane is on the body
+            const uint32_t m = min(32u, n - k0);
+            for (uint32_t j = 0; j < m; ++j)
+            {
+                const uint32_t ja = __shfl_sync(0xffffffffu, r.x, j), jb = __shfl_sync(0xffffffffu, r.y, j);
+                const uint32_t jl = __shfl_sync(0xffffffffu, l, j);
+                const bool on_a = da && (ja == r.x || jb == r.x), on_b = db && (ja == r.y || jb == r.y);
+                if (j < lane && (on_a || on_b))
+                    l = max(l, jl + 1u);
+                if (j > lane)
+                {
+                    last_a = last_a && !on_a;
+                    last_b = last_b && !on_b;
+                }
+            }
+            __syncwarp();
+            if (lane < m)
+            {
+                lvl[k0 + lane] = l;
+                top = max(top, l + 1u);
+                if (last_a)
+                    last[a] = l + 1u;
+                if (last_b)
+                    last[b] = l + 1u;
+            }
+            __syncwarp();
+        }
+        return __reduce_max_sync(0xffffffffu, top);
+    }
+
+    // The reference's order as levels.  The reference relaxes its contact
+    // list one entry after another (World.hpp:168-180); entries that share no
+    // dynamic body touch disjoint state, so each may run as soon as the
+    // earlier entries on its two bodies have.  The active candidates
+    // (S.alist[0, n_act), in list order) are bucketed by that level, and the
+    // solves relax a level at a time with the team, with the same bits as the
+    // serial walk.  `last` is a word per body of scratch; `book` the team's
+    // shared words (136) when it has them.  Level l ends up in
+    // [off[l], off[l + 1]) of S.corder, where off is `book` or, with more
+    // levels than that holds, S.loff (level_offsets).
+    // The walk on one thread, a dependent global load for every candidate
+    // whether it contacts or not, was 94 % of a step.  512 bodies, 10
+    // substeps, FP64: 13.5 ms a step with it, 1.22 ms with the levels; 96
+    // worlds of 8 to 128 bodies, 2 steps: 6.87 against 2.83 ms.
+    constexpr uint32_t kBookLevels = 130;
+
+    template <class T, class P, class Team>
+    __device__ void schedule_levels(const Engine<T, P> &E, const Team &tm, const WorldDev &W, const Scr<T, P> &S,
+                                    uint32_t n_act, uint32_t *last, uint32_t *book)
+    {
+        const uint8_t *type = E.B.type + W.body_off;
+        for (uint32_t b = tm.rank(); b < W.n_bodies; b += tm.size())
+            last[b] = 0u;
+        for (uint32_t q = tm.rank(); q < n_act; q += tm.size())
+        {
+            const Cand cd = S.cand[S.alist[q]];
+            S.lrec[q] = make_uint2(cd.ba | (type[cd.ba] == kDynamic ? 0x80000000u : 0u),
+                                   cd.bb | (type[cd.bb] == kDynamic ? 0x80000000u : 0u));
+        }
+        tm.sync();
+        if (tm.rank() < 32)
+        {
+            const uint32_t n = levels_warp(S.lrec, n_act, last, S.act);
+            if (tm.leader())
+                S.misc[kMiscNColors] = n;
+        }
+        tm.sync();
+        const uint32_t n_lvl = S.misc[kMiscNColors];
+        uint32_t *off = book && n_lvl <= kBookLevels ? book : S.loff;
+        for (uint32_t l = tm.rank(); l <= n_lvl; l += tm.size())
+            off[l] = 0u;
+        if (book && tm.leader())
+            book[132] = n_lvl;
+        tm.sync();
+        for (uint32_t q = tm.rank(); q < n_act; q += tm.size())
+            atomicAdd(&off[1u + S.act[q]], 1u);
+        tm.sync();
+        // counts to first slots; as the slots fill, each becomes its end
+        if (tm.rank() < 32)
+        {
+            uint32_t run = 0;
+            for (uint32_t l0 = 0; l0 < n_lvl; l0 += 32)
+            {
+                const uint32_t l = l0 + lane_id();
+                const uint32_t v = l < n_lvl ? off[1u + l] : 0u;
+                const uint32_t inc = warp_incl_scan(v);
+                if (l < n_lvl)
+                    off[1u + l] = run + inc - v;
+                run += __shfl_sync(0xffffffffu, inc, 31);
+            }
+        }
+        tm.sync();
+        for (uint32_t q = tm.rank(); q < n_act; q += tm.size())
+        {
+            const uint32_t c = S.alist[q];
+            S.corder[atomicAdd(&off[1u + S.act[q]], 1u)] = c;
+            prefetch_l2_range(S.cc + c, sizeof(CandContacts<T, P>));
+        }
+        tm.sync();
+    }
+
+    // Offsets and number of the levels schedule_levels left.
+    template <class T, class P>
+    __device__ __forceinline__ const uint32_t *level_offsets(const Scr<T, P> &S, const uint32_t *book, uint32_t &n)
+    {
+        n = book ? book[132] : S.misc[kMiscNColors];
+        return book && n <= kBookLevels ? book : S.loff;
+    }
+
     // Colouring of the candidates that produced contact rows in this substep
-    // (the others have nothing to relax), in rounds:
-    // * up to kGridWorldBodies bodies, Jones-Plassmann: a candidate takes the
-    //   lowest colour free on both of its dynamic bodies once it holds the
-    //   highest priority among the uncoloured candidates sharing them.  A
-    //   body gets at most one colour a round, so a body with d contacts takes
-    //   d rounds or more;
-    // * larger worlds, claims: every uncoloured candidate picks one colour
-    //   free on both bodies (hashed among the lowest few) and claims that
-    //   (body, colour) slot on each; the highest claim on both slots wins.
-    //   Many contacts of one body are coloured per round: on tangled chains
-    //   (contacts up to 53 per body) 8 rounds instead of more than 96.
-    // Both are deterministic (priorities are hashes of the candidate index).
+    // (the others have nothing to relax) on the grid, in rounds of claims:
+    // every uncoloured candidate picks one colour free on both bodies (hashed
+    // among the lowest few) and claims that (body, colour) slot on each; the
+    // highest claim on both slots wins.  Many contacts of one body are
+    // coloured per round: on tangled chains (contacts up to 53 per body) 8
+    // rounds, where one colour a body and round took more than 96.
+    // Deterministic (priorities are hashes of the candidate index).
     // Candidates whose bodies have used all 64 colours, or still uncoloured
     // after kMaxColorRounds, go to the serial colour; idle candidates get
     // kColorIdle and are not bucketed.  Returns the number of regular
     // colours; corder / colour offsets are filled.
     // Second-level colours for the overflow bucket [coff[64], coff[65]) of
     // corder: the team leader colours its candidates first-fit in order on
-    // a second set of body masks (bprio, free after the Jones-Plassmann
+    // a second set of body masks (bprio, free after the claim
     // rounds), and the bucket is reordered by those colours, so that the
     // solves can relax it colour by colour (kMiscC2Off) instead of on one
     // thread; entry 64 keeps what still does not fit.  The bucket comes
@@ -911,37 +1066,23 @@ namespace rbps_gpu
         tm.sync();
     }
 
-    template <class T, class P, class Team>
-    __device__ uint32_t color_active(const Engine<T, P> &E, const Team &tm, const WorldDev &W, const Scr<T, P> &S,
+    template <class T, class P>
+    __device__ uint32_t color_active(const Engine<T, P> &E, const GridTeam &tm, const WorldDev &W, const Scr<T, P> &S,
                                      uint32_t n_cand, BlockShared &sh)
     {
         uint32_t *misc = S.misc;
-        // compact the active candidates into alist
-        for (uint32_t c = tm.rank(); c < n_cand; c += tm.size())
-            S.act[c] = S.cc[c].n > 0 ? 1u : 0u;
         for (uint32_t b = tm.rank(); b < W.n_bodies; b += tm.size())
         {
             S.bmask[b] = 0ull;
             S.bprio[b] = 0ull;
         }
-        const bool by_claim = W.n_bodies > kGridWorldBodies;
-        if (by_claim)
-            for (uint32_t x = tm.rank(); x < W.n_bodies * 64u; x += tm.size())
-                S.claim[x] = 0ull;
+        for (uint32_t x = tm.rank(); x < W.n_bodies * 64u; x += tm.size())
+            S.claim[x] = 0ull;
         for (uint32_t x = tm.rank(); x < kMaxColorRounds + 2 * 66; x += tm.size())
             misc[kMiscCCount + x] = 0u;
-        tm.sync();
-        const uint32_t n_act = team_excl_scan(tm, S.act, S.act, n_cand, S.tile_sums, sh);
-        for (uint32_t c = tm.rank(); c < n_cand; c += tm.size())
-        {
-            if (S.cc[c].n > 0)
-                S.alist[S.act[c]] = c;
-            S.color[c] = S.cc[c].n > 0 ? 0xffffffffu : kColorIdle;
-        }
-        tm.sync();
+        const uint32_t n_act = compact_grid(tm, S, n_cand, sh);
         const uint8_t *type = E.B.type + W.body_off;
         uint32_t round = 1;
-        if (by_claim)
         {
             // uncoloured contacts per body (bprio's words reused as counters)
             uint32_t *ucnt = (uint32_t *)S.bprio;
@@ -1027,56 +1168,6 @@ namespace rbps_gpu
                 if (misc[kMiscLeft + round - 1] == 0u)
                     break;
             }
-        }
-        for (; !by_claim && round <= kMaxColorRounds && n_act; ++round)
-        {
-            for (uint32_t q = tm.rank(); q < n_act; q += tm.size())
-            {
-                const uint32_t c = S.alist[q];
-                if (S.color[c] != 0xffffffffu)
-                    continue;
-                const Cand cd = S.cand[c];
-                const unsigned long long val = ((unsigned long long)round << 56) |
-                                               ((unsigned long long)(hash32(c) & 0xffffffu) << 32) | c;
-                if (type[cd.ba] == kDynamic)
-                    atomicMax(&S.bprio[cd.ba], val);
-                if (type[cd.bb] == kDynamic)
-                    atomicMax(&S.bprio[cd.bb], val);
-            }
-            tm.sync();
-            for (uint32_t q = tm.rank(); q < n_act; q += tm.size())
-            {
-                const uint32_t c = S.alist[q];
-                if (S.color[c] != 0xffffffffu)
-                    continue;
-                const Cand cd = S.cand[c];
-                const unsigned long long val = ((unsigned long long)round << 56) |
-                                               ((unsigned long long)(hash32(c) & 0xffffffu) << 32) | c;
-                const bool da = type[cd.ba] == kDynamic, db = type[cd.bb] == kDynamic;
-                const bool won = (!da || S.bprio[cd.ba] == val) && (!db || S.bprio[cd.bb] == val);
-                if (!won)
-                {
-                    atomicAdd(&misc[kMiscLeft + round - 1], 1u);
-                    continue;
-                }
-                const unsigned long long used = (da ? S.bmask[cd.ba] : 0ull) | (db ? S.bmask[cd.bb] : 0ull);
-                uint32_t col;
-                if (used == ~0ull)
-                    col = kColorSerial;
-                else
-                {
-                    col = (uint32_t)(__ffsll((long long)~used) - 1);
-                    const unsigned long long bit = 1ull << col;
-                    if (da)
-                        S.bmask[cd.ba] |= bit;
-                    if (db)
-                        S.bmask[cd.bb] |= bit;
-                }
-                S.color[c] = col;
-            }
-            tm.sync();
-            if (misc[kMiscLeft + round - 1] == 0u)
-                break;
         }
         if (round > kMaxColorRounds)
         {
@@ -1392,14 +1483,6 @@ namespace rbps_gpu
         slot_pair(S, book, q, c, ba, bb);
     }
 
-    // Asks L2 for every 128-byte line of [p, p + bytes) (prefetch.global.L2).
-    __device__ __forceinline__ void prefetch_l2_range(const void *p, size_t bytes)
-    {
-        const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-        for (uintptr_t l = a & ~uintptr_t(127); l < a + bytes; l += 128)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(l));
-    }
-
     // ------------------------------------------------------------ the step
     // World::step (World.hpp:192-212) as phases.  Every phase ends with a
     // team barrier and keeps its state in the world's scratch slice, so each
@@ -1452,20 +1535,23 @@ namespace rbps_gpu
         clk.mark(kPhNarrow);
     }
 
-    // Colouring of the contacting candidates (colored mode), then integrate
-    // (Body.cpp:18-39).
+    // Colouring of the contacting candidates (their levels in reference
+    // order), then integrate (Body.cpp:18-39).
     template <class T, class P, class Team>
     __device__ void phase_color_integrate(const Engine<T, P> &E, const Team &tm, uint32_t w, BlockShared &sh)
     {
         const WorldDev W = E.worlds[w];
         const Scr<T, P> S = world_scratch(E, W);
         PhaseClock clk(prof_slots(E, tm, w), false);
+        const uint32_t n_cand = S.misc[kMiscNCand];
         if (E.solve_mode == 1)
         {
-            const uint32_t nc = color_active(E, tm, W, S, S.misc[kMiscNCand], sh);
+            const uint32_t nc = color_active(E, tm, W, S, n_cand, sh);
             if (tm.leader() && nc > S.misc[kMiscMaxColors])
                 S.misc[kMiscMaxColors] = nc;
         }
+        else
+            schedule_levels(E, tm, W, S, compact_grid(tm, S, n_cand, sh), (uint32_t *)S.bmask, nullptr);
         clk.mark(kPhColor);
         for (uint32_t b = tm.rank(); b < W.n_bodies; b += tm.size())
             integrate_body(E.B, W.body_off + b, E.h);
@@ -1527,7 +1613,9 @@ namespace rbps_gpu
             tm.sync();
     }
 
-    template <class T, class P, class Team>
+    // Ref: the reference's order, level by level (schedule_levels), else
+    // colour by colour.
+    template <bool Ref, class T, class P, class Team>
     __device__ void phase_position_on(const Engine<T, P> &E, const Team &tm, uint32_t w, const Bodies<T, P> &B,
                                       uint32_t boff, const uint32_t *book = nullptr, const uint2 *slots = nullptr)
     {
@@ -1535,34 +1623,27 @@ namespace rbps_gpu
         const Scr<T, P> S = world_scratch(E, W);
         PhaseClock clk(prof_slots(E, tm, w), false);
         const uint32_t shift = W.body_off - boff; // joint body ids are batch-global
-        const uint32_t n_cand = S.misc[kMiscNCand];
-        if (E.solve_mode != 1)
+        if constexpr (Ref)
         {
-            if (tm.leader())
-            {
-                for (uint32_t c = 0; c < n_cand; ++c)
-                {
+            uint32_t n_lvl;
+            const uint32_t *loff = level_offsets(S, book, n_lvl);
+            if constexpr (std::is_same<Team, GridTeam>::value)
+                sweep_colors(tm, loff, n_lvl, [&](uint32_t q) {
+                    const uint32_t c = S.corder[q];
                     const Cand cd = S.cand[c];
                     solve_pair_position(B, E.inv_h, boff + cd.ba, boff + cd.bb, S.cc[c]);
-                }
-                for (uint32_t j = 0; j < W.n_joints; ++j)
+                });
+            else
+                for (uint32_t l = 0; l < n_lvl; ++l)
                 {
-                    Joint<T> jt = E.joints[W.joint_off + j];
-                    jt.b1 -= shift;
-                    jt.b2 -= shift;
-                    joint_errors(B, jt, joint_rows(E, jt), E.h);
-                    E.joints[W.joint_off + j].target_pos = jt.target_pos;
+                    for (uint32_t q = loff[l] + tm.rank(); q < loff[l + 1]; q += tm.size())
+                    {
+                        const uint32_t c = S.corder[q];
+                        const Cand cd = S.cand[c];
+                        solve_pair_position(B, E.inv_h, boff + cd.ba, boff + cd.bb, S.cc[c]);
+                    }
+                    tm.sync();
                 }
-                for (uint32_t j = 0; j < W.n_joints; ++j)
-                {
-                    Joint<T> jt = E.joints[W.joint_off + j];
-                    jt.b1 -= shift;
-                    jt.b2 -= shift;
-                    solve_joint_rows(B, jt, joint_rows(E, jt), E.inv_h);
-                }
-            }
-            tm.sync();
-            clk.mark(kPhContactPos); // reference order: contacts and joints in one phase
         }
         else
         {
@@ -1598,33 +1679,33 @@ namespace rbps_gpu
                     }
                 tm.sync();
             }
-            clk.mark(kPhContactPos);
-            if (W.n_joints)
+        }
+        clk.mark(kPhContactPos);
+        if (W.n_joints)
+        {
+            for (uint32_t j = tm.rank(); j < W.n_joints; j += tm.size())
             {
-                for (uint32_t j = tm.rank(); j < W.n_joints; j += tm.size())
+                Joint<T> jt = E.joints[W.joint_off + j];
+                jt.b1 -= shift;
+                jt.b2 -= shift;
+                joint_errors(B, jt, joint_rows(E, jt), E.h);
+                E.joints[W.joint_off + j].target_pos = jt.target_pos;
+            }
+            tm.sync();
+            const uint32_t *jco = E.jcolor_off + W.jc_off;
+            for (uint32_t jc = 0; jc < W.n_jcolors; ++jc)
+            {
+                for (uint32_t q = jco[jc] + tm.rank(); q < jco[jc + 1]; q += tm.size())
                 {
-                    Joint<T> jt = E.joints[W.joint_off + j];
+                    Joint<T> jt = E.joints[W.joint_off + E.jorder[q]];
                     jt.b1 -= shift;
                     jt.b2 -= shift;
-                    joint_errors(B, jt, joint_rows(E, jt), E.h);
-                    E.joints[W.joint_off + j].target_pos = jt.target_pos;
+                    solve_joint_rows(B, jt, joint_rows(E, jt), E.inv_h);
                 }
                 tm.sync();
-                const uint32_t *jco = E.jcolor_off + W.jc_off;
-                for (uint32_t jc = 0; jc < W.n_jcolors; ++jc)
-                {
-                    for (uint32_t q = jco[jc] + tm.rank(); q < jco[jc + 1]; q += tm.size())
-                    {
-                        Joint<T> jt = E.joints[W.joint_off + E.jorder[q]];
-                        jt.b1 -= shift;
-                        jt.b2 -= shift;
-                        solve_joint_rows(B, jt, joint_rows(E, jt), E.inv_h);
-                    }
-                    tm.sync();
-                }
             }
-            clk.mark(kPhJointPos);
         }
+        clk.mark(kPhJointPos);
         for (uint32_t b = tm.rank(); b < W.n_bodies; b += tm.size())
             update_velocity_body(B, boff + b, E.inv_h);
         tm.sync();
@@ -1634,11 +1715,14 @@ namespace rbps_gpu
     template <class T, class P, class Team>
     __device__ void phase_position(const Engine<T, P> &E, const Team &tm, uint32_t w)
     {
-        phase_position_on(E, tm, w, E.B, E.worlds[w].body_off);
+        if (E.solve_mode == 1)
+            phase_position_on<false>(E, tm, w, E.B, E.worlds[w].body_off);
+        else
+            phase_position_on<true>(E, tm, w, E.B, E.worlds[w].body_off);
     }
 
     // Velocity solve (World.hpp:176-180): restitution / friction, joint damping.
-    template <class T, class P, class Team>
+    template <bool Ref, class T, class P, class Team>
     __device__ void phase_velocity_on(const Engine<T, P> &E, const Team &tm, uint32_t w, const Bodies<T, P> &B,
                                       uint32_t boff, const uint32_t *book = nullptr, const uint2 *slots = nullptr)
     {
@@ -1646,25 +1730,27 @@ namespace rbps_gpu
         const Scr<T, P> S = world_scratch(E, W);
         PhaseClock clk(prof_slots(E, tm, w), false);
         const uint32_t shift = W.body_off - boff;
-        if (E.solve_mode != 1)
+        if constexpr (Ref)
         {
-            if (tm.leader())
-            {
-                const uint32_t n_cand = S.misc[kMiscNCand];
-                for (uint32_t c = 0; c < n_cand; ++c)
-                {
+            uint32_t n_lvl;
+            const uint32_t *loff = level_offsets(S, book, n_lvl);
+            if constexpr (std::is_same<Team, GridTeam>::value)
+                sweep_colors(tm, loff, n_lvl, [&](uint32_t q) {
+                    const uint32_t c = S.corder[q];
                     const Cand cd = S.cand[c];
                     solve_pair_velocity(B, E.h, boff + cd.ba, boff + cd.bb, S.cc[c]);
-                }
-                for (uint32_t j = 0; j < W.n_joints; ++j)
+                });
+            else
+                for (uint32_t l = 0; l < n_lvl; ++l)
                 {
-                    Joint<T> jt = E.joints[W.joint_off + j];
-                    jt.b1 -= shift;
-                    jt.b2 -= shift;
-                    joint_damping(B, jt, E.h);
+                    for (uint32_t q = loff[l] + tm.rank(); q < loff[l + 1]; q += tm.size())
+                    {
+                        const uint32_t c = S.corder[q];
+                        const Cand cd = S.cand[c];
+                        solve_pair_velocity(B, E.h, boff + cd.ba, boff + cd.bb, S.cc[c]);
+                    }
+                    tm.sync();
                 }
-            }
-            tm.sync();
         }
         else
         {
@@ -1698,18 +1784,18 @@ namespace rbps_gpu
                     }
                 tm.sync();
             }
-            const uint32_t *jco = E.jcolor_off + W.jc_off;
-            for (uint32_t jc = 0; jc < W.n_jcolors; ++jc)
+        }
+        const uint32_t *jco = E.jcolor_off + W.jc_off;
+        for (uint32_t jc = 0; jc < W.n_jcolors; ++jc)
+        {
+            for (uint32_t q = jco[jc] + tm.rank(); q < jco[jc + 1]; q += tm.size())
             {
-                for (uint32_t q = jco[jc] + tm.rank(); q < jco[jc + 1]; q += tm.size())
-                {
-                    Joint<T> jt = E.joints[W.joint_off + E.jorder[q]];
-                    jt.b1 -= shift;
-                    jt.b2 -= shift;
-                    joint_damping(B, jt, E.h);
-                }
-                tm.sync();
+                Joint<T> jt = E.joints[W.joint_off + E.jorder[q]];
+                jt.b1 -= shift;
+                jt.b2 -= shift;
+                joint_damping(B, jt, E.h);
             }
+            tm.sync();
         }
         clk.mark(kPhVelSolve);
     }
@@ -1717,7 +1803,10 @@ namespace rbps_gpu
     template <class T, class P, class Team>
     __device__ void phase_velocity(const Engine<T, P> &E, const Team &tm, uint32_t w)
     {
-        phase_velocity_on(E, tm, w, E.B, E.worlds[w].body_off);
+        if (E.solve_mode == 1)
+            phase_velocity_on<false>(E, tm, w, E.B, E.worlds[w].body_off);
+        else
+            phase_velocity_on<true>(E, tm, w, E.B, E.worlds[w].body_off);
     }
 
     // Statistics and parity dumps of the last substep.
@@ -1826,36 +1915,6 @@ namespace rbps_gpu
     }
 
     template <class T, class P>
-    __global__ void __launch_bounds__(kMaxBlock) k_phase_narrow(const Engine<T, P> E, uint32_t ctr)
-    {
-        BlockTeam tm;
-        each_small_world(E.small_worlds, E.n_small, E.work_counter + ctr, [&](uint32_t w) { phase_narrow(E, tm, w); });
-    }
-
-    template <class T, class P>
-    __global__ void __launch_bounds__(kMaxBlock) k_phase_color(const Engine<T, P> E, uint32_t ctr)
-    {
-        __shared__ BlockShared sh;
-        BlockTeam tm;
-        each_small_world(E.small_worlds, E.n_small, E.work_counter + ctr,
-                         [&](uint32_t w) { phase_color_integrate(E, tm, w, sh); });
-    }
-
-    template <class T, class P>
-    __global__ void __launch_bounds__(kMaxBlock) k_phase_position(const Engine<T, P> E, uint32_t ctr)
-    {
-        BlockTeam tm;
-        each_small_world(E.small_worlds, E.n_small, E.work_counter + ctr, [&](uint32_t w) { phase_position(E, tm, w); });
-    }
-
-    template <class T, class P>
-    __global__ void __launch_bounds__(kMaxBlock) k_phase_velocity(const Engine<T, P> E, uint32_t ctr)
-    {
-        BlockTeam tm;
-        each_small_world(E.small_worlds, E.n_small, E.work_counter + ctr, [&](uint32_t w) { phase_velocity(E, tm, w); });
-    }
-
-    template <class T, class P>
     __global__ void __launch_bounds__(kMaxBlock) k_phase_stats(const Engine<T, P> E, uint32_t ctr)
     {
         BlockTeam tm;
@@ -1889,29 +1948,8 @@ namespace rbps_gpu
         }
     }
 
-    // Enqueues one step of every small world: 2 + 4 * substeps phase kernels
-    // (work counters ctr_base .. ctr_base + 1 + 4 * substeps must be zero).
-    template <class T, class P>
-    cudaError_t launch_step_phases(const Engine<T, P> &e, const PhaseLaunch &pl, cudaStream_t stream)
-    {
-        uint32_t ctr = 0;
-        k_phase_frame<T, P><<<pl.grid[kKFrame], pl.block[kKFrame], 0, stream>>>(e, ctr++);
-        for (int s = 0; s < e.substeps; ++s)
-        {
-            if (e.gjk_list)
-                cudaMemsetAsync(e.gjk_count, 0, 4, stream);
-            k_phase_narrow<T, P><<<pl.grid[kKNarrow], pl.block[kKNarrow], 0, stream>>>(e, ctr++);
-            launch_gjk(e, stream);
-            k_phase_color<T, P><<<pl.grid[kKColor], pl.block[kKColor], 0, stream>>>(e, ctr++);
-            k_phase_position<T, P><<<pl.grid[kKPosition], pl.block[kKPosition], 0, stream>>>(e, ctr++);
-            k_phase_velocity<T, P><<<pl.grid[kKVelocity], pl.block[kKVelocity], 0, stream>>>(e, ctr++);
-        }
-        k_phase_stats<T, P><<<pl.grid[kKStats], pl.block[kKStats], 0, stream>>>(e, ctr++);
-        return cudaGetLastError();
-    }
-
-    // ------------------------------------------------- batched colored pipeline
-    // Colored mode over the small worlds, per step:
+    // --------------------------------------------------------- batched pipeline
+    // The small worlds, per step:
     //   k_phase_frame    one CTA per world: SAP update / sort / sweep, candidates
     //   k_flat_prefix    candidate prefix over the worlds
     //   k_type_count / k_type_scan / k_type_scatter
@@ -1921,10 +1959,11 @@ namespace rbps_gpu
     //   k_flat_narrow    one thread per candidate, in shape-pair order; the
     //                    box-box class in k_flat_narrow_boxbox
     //   k_substep        one CTA per large world, one warp per other world:
-    //                    greedy colouring of the contacting candidates, integrate,
-    //                    position solve (colour by colour, joint errors, joint
-    //                    colours), velocity update, velocity solve -- worlds
-    //                    progress independently on their own team barriers
+    //                    greedy colouring of the contacting candidates (in
+    //                    reference order their levels), integrate, position
+    //                    solve (colour by colour, joint errors, joint colours),
+    //                    velocity update, velocity solve -- worlds progress
+    //                    independently on their own team barriers
     // and last k_phase_stats.
 
     // Candidate prefix over the small worlds (one CTA).
@@ -2285,6 +2324,23 @@ namespace rbps_gpu
         return kept + fresh;
     }
 
+    // The levels of world w's contacting candidates (schedule_levels), and
+    // its contact rows counted.
+    template <class T, class P, class Team>
+    __device__ void level_world(const Engine<T, P> &E, const Team &tm, uint32_t w, uint32_t *last, uint32_t *book,
+                                ScanShared &sh)
+    {
+        const WorldDev W = E.worlds[w];
+        const Scr<T, P> S = world_scratch(E, W);
+        uint32_t rows = 0;
+        if (tm.leader())
+            S.misc[kMiscNContacts] = 0u;
+        const uint32_t n_act = compact_active(tm, S, S.misc[kMiscNCand], sh, &rows);
+        if (rows) // after the compaction's closing barrier, so after the reset
+            atomicAdd(S.misc + kMiscNContacts, rows);
+        schedule_levels(E, tm, W, S, n_act, last, book);
+    }
+
     // Greedy colouring of the world's contacting candidates: in candidate
     // order, each takes the lowest colour free on both of its dynamic bodies
     // (kColorSerial once a body has used all 64).  The team leader colours
@@ -2556,6 +2612,10 @@ namespace rbps_gpu
 #ifndef RBPS_SUBSTEP_MIN_BLOCKS
 #define RBPS_SUBSTEP_MIN_BLOCKS 4
 #endif
+// In double a pair's two bodies alone take 104 registers: two CTAs (255).
+#ifndef RBPS_SUBSTEP_MIN_BLOCKS_F64
+#define RBPS_SUBSTEP_MIN_BLOCKS_F64 2
+#endif
     // The rest of a substep for every small world: colouring, integrate
     // (Body.cpp:18-39), position solve + velocity update, velocity solve.
     // The largest worlds (the first n_block_worlds of the list) get a whole
@@ -2661,7 +2721,7 @@ namespace rbps_gpu
             st.n_cand = misc[kMiscNCand];
             st.n_contacts = misc[kMiscNContacts];
             st.n_colors = misc[kMiscMaxColors];
-            st.n_serial = misc[kMiscCOff + kColorSerial + 1] - misc[kMiscCOff + kColorSerial];
+            st.n_serial = E.solve_mode == 1 ? misc[kMiscCOff + kColorSerial + 1] - misc[kMiscCOff + kColorSerial] : 0u;
             st.n_gjk = misc[kMiscNGjk];
             st.pad_[0] = st.pad_[1] = 0;
             E.stats[w] = st;
@@ -2674,7 +2734,7 @@ namespace rbps_gpu
     // velocity update, velocity solve.  With `smem` (room for `cap` bodies)
     // and a world that fits, the bodies live in shared memory for the whole
     // substep and are written back once.
-    template <class T, class P, class Team>
+    template <bool Ref, class T, class P, class Team>
     __device__ void substep_world(const Engine<T, P> &E, const Team &tm, uint32_t w, unsigned char *smem,
                                   uint32_t cap, ScanShared &sh)
     {
@@ -2693,10 +2753,13 @@ namespace rbps_gpu
         else
             mask = world_scratch(E, W).bmask;
         PhaseClock clk(prof_slots(E, tm, w), false);
-        // the pose copy is not loaded yet: its first words serve the
-        // colouring as per-body scratch
-        greedy_color_world(E, tm, w, mask, sh, book, stage, local ? reinterpret_cast<uint32_t *>(V.pos) : nullptr, slots,
-                           cap * SmemWorld<T, P>::kSlotsPerBody);
+        if constexpr (Ref)
+            level_world(E, tm, w, reinterpret_cast<uint32_t *>(mask), book, sh);
+        else
+            // the pose copy is not loaded yet: its first words serve the
+            // colouring as per-body scratch
+            greedy_color_world(E, tm, w, mask, sh, book, stage, local ? reinterpret_cast<uint32_t *>(V.pos) : nullptr,
+                               slots, cap * SmemWorld<T, P>::kSlotsPerBody);
         clk.mark(kPhColor);
         // integrate (Body.cpp:18-39); a world in shared memory is loaded
         // into its copy by the same pass
@@ -2707,8 +2770,8 @@ namespace rbps_gpu
                 integrate_body(V, boff + b, E.h);
         tm.sync();
         clk.mark(kPhIntegrate);
-        phase_position_on(E, tm, w, V, boff, book, slots);
-        phase_velocity_on(E, tm, w, V, boff, book, slots);
+        phase_position_on<Ref>(E, tm, w, V, boff, book, slots);
+        phase_velocity_on<Ref>(E, tm, w, V, boff, book, slots);
         if (local)
         {
             const Bodies<T, P> &G = E.B;
@@ -2744,15 +2807,16 @@ namespace rbps_gpu
     // barrier is the team's own.  Dynamic shared memory: E.smem_cap_block
     // bodies for a CTA world, E.smem_cap_pair for each of two half-CTA
     // worlds, or E.smem_cap_warp for each of four warp worlds.
-    template <class T, class P>
-    __global__ void __launch_bounds__(128, RBPS_SUBSTEP_MIN_BLOCKS) k_substep(const Engine<T, P> E)
+    template <class T, class P, bool Ref>
+    __global__ void __launch_bounds__(128, sizeof(T) == 8 ? RBPS_SUBSTEP_MIN_BLOCKS_F64 : RBPS_SUBSTEP_MIN_BLOCKS)
+        k_substep(const Engine<T, P> E)
     {
         __shared__ ScanShared sh; // the colouring's compaction scans are all the teams need
         extern __shared__ __align__(16) unsigned char smem[];
         if (blockIdx.x < E.n_block_worlds)
         {
             BlockTeam tm;
-            substep_world(E, tm, E.small_worlds[blockIdx.x], smem, E.smem_cap_block, sh);
+            substep_world<Ref>(E, tm, E.small_worlds[blockIdx.x], smem, E.smem_cap_block, sh);
             return;
         }
         const uint32_t pair_ctas = (E.n_pair_worlds + 1) / 2;
@@ -2765,7 +2829,7 @@ namespace rbps_gpu
             if (k >= E.n_pair_worlds)
                 return;
             PairTeam tm;
-            substep_world(E, tm, E.small_worlds[E.n_block_worlds + k],
+            substep_world<Ref>(E, tm, E.small_worlds[E.n_block_worlds + k],
                           smem + (threadIdx.x >> 6) * SmemWorld<T, P>::bytes(E.smem_cap_pair), E.smem_cap_pair, sh);
             return;
         }
@@ -2773,8 +2837,54 @@ namespace rbps_gpu
         if (q >= E.n_small)
             return;
         WarpTeam tm;
-        substep_world(E, tm, E.small_worlds[q], smem + warp_id() * SmemWorld<T, P>::bytes(E.smem_cap_warp),
+        substep_world<Ref>(E, tm, E.small_worlds[q], smem + warp_id() * SmemWorld<T, P>::bytes(E.smem_cap_warp),
                       E.smem_cap_warp, sh);
+    }
+
+    // A substep in the reference's order in float, one CTA per world and one
+    // launch per phase on the batch arrays.  k_substep would take it too, but
+    // which products of a contact row contract into FMAs is the compiler's
+    // choice for each kernel, and a settled pile carries a last bit to whole
+    // metres in a second: these two kernels, with both solve modes in them
+    // and the level loop written out, keep the results float worlds have had.
+    // (Double has no contraction and runs in k_substep.)
+    template <class T, class P>
+    __global__ void __launch_bounds__(kMaxBlock) k_ref_levels(const Engine<T, P> E)
+    {
+        __shared__ ScanShared sh;
+        BlockTeam tm;
+        const uint32_t w = E.small_worlds[blockIdx.x];
+        const WorldDev W = E.worlds[w];
+        PhaseClock clk(prof_slots(E, tm, w), false);
+        level_world(E, tm, w, (uint32_t *)world_scratch(E, W).bmask, nullptr, sh);
+        clk.mark(kPhColor);
+        for (uint32_t b = tm.rank(); b < W.n_bodies; b += tm.size())
+            integrate_body(E.B, W.body_off + b, E.h);
+        tm.sync();
+        clk.mark(kPhIntegrate);
+    }
+
+    template <class T, class P>
+    __global__ void __launch_bounds__(kMaxBlock) k_ref_position(const Engine<T, P> E)
+    {
+        BlockTeam tm;
+        const uint32_t w = E.small_worlds[blockIdx.x];
+        phase_position(E, tm, w);
+    }
+
+    template <class T, class P>
+    __global__ void __launch_bounds__(kMaxBlock) k_ref_velocity(const Engine<T, P> E)
+    {
+        BlockTeam tm;
+        const uint32_t w = E.small_worlds[blockIdx.x];
+        phase_velocity(E, tm, w);
+        if (E.stats_in_substep)
+        {
+            PhaseClock clk(prof_slots(E, tm, w), false);
+            substep_stats(E, tm, w, E.B, E.worlds[w].body_off);
+            clk.mark(kPhStats);
+            clk.finish();
+        }
     }
 
     // Opens k_substep to `bytes` of dynamic shared memory.
@@ -2784,13 +2894,18 @@ namespace rbps_gpu
         // the attribute belongs to the kernel on the current device, shared
         // by every batch there: only ever raise it, or a batch created later
         // with smaller worlds would make an earlier one's launches fail
-        cudaFuncAttributes fa;
-        cudaError_t rc = cudaFuncGetAttributes(&fa, k_substep<T, P>);
-        if (rc != cudaSuccess)
+        auto open = [bytes](auto *kernel) {
+            cudaFuncAttributes fa;
+            cudaError_t rc = cudaFuncGetAttributes(&fa, kernel);
+            if (rc == cudaSuccess && (size_t)fa.maxDynamicSharedSizeBytes < bytes)
+                rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
             return rc;
-        if ((size_t)fa.maxDynamicSharedSizeBytes >= bytes)
-            return cudaSuccess;
-        return cudaFuncSetAttribute(k_substep<T, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        };
+        cudaError_t rc = open(k_substep<T, P, false>);
+        if constexpr (sizeof(T) == 8)
+            if (rc == cudaSuccess)
+                rc = open(k_substep<T, P, true>);
+        return rc;
     }
 
     template <class T, class P>
@@ -2815,17 +2930,17 @@ namespace rbps_gpu
         {
             if (e.gjk_list)
                 cudaMemsetAsync(e.gjk_count, 0, 4, stream);
-            if (fl.side && s < 8)
+            if (fl.side)
             {
                 // the two narrowphase kernels touch disjoint candidates: run
                 // them side by side (a fork / join the graph capture keeps)
-                cudaEventRecord(fl.fork[s], stream);
-                cudaStreamWaitEvent(fl.side, fl.fork[s], 0);
+                cudaEventRecord(fl.fork, stream);
+                cudaStreamWaitEvent(fl.side, fl.fork, 0);
                 k_flat_narrow_boxbox<T, P><<<fl.grid_narrow, kMaxBlock, 0, fl.side>>>(e);
                 k_flat_narrow_other<T, P><<<fl.grid_narrow, kMaxBlock, 0, fl.side>>>(e);
-                cudaEventRecord(fl.join[s], fl.side);
+                cudaEventRecord(fl.join, fl.side);
                 k_flat_narrow<T, P><<<fl.grid_narrow, kMaxBlock, 0, stream>>>(e);
-                cudaStreamWaitEvent(stream, fl.join[s], 0);
+                cudaStreamWaitEvent(stream, fl.join, 0);
             }
             else
             {
@@ -2834,7 +2949,17 @@ namespace rbps_gpu
                 k_flat_narrow_other<T, P><<<fl.grid_narrow, kMaxBlock, 0, stream>>>(e);
             }
             launch_gjk(e, stream);
-            k_substep<T, P><<<fl.grid_solve, 128, fl.substep_smem, stream>>>(s + 1 == e.substeps ? el : e);
+            const Engine<T, P> &es = s + 1 == e.substeps ? el : e;
+            if (e.solve_mode == 1)
+                k_substep<T, P, false><<<fl.grid_solve, 128, fl.substep_smem, stream>>>(es);
+            else if constexpr (sizeof(T) == 8)
+                k_substep<T, P, true><<<fl.grid_solve, 128, fl.substep_smem, stream>>>(es);
+            else
+            {
+                k_ref_levels<T, P><<<e.n_small, 128, 0, stream>>>(es);
+                k_ref_position<T, P><<<e.n_small, 128, 0, stream>>>(es);
+                k_ref_velocity<T, P><<<e.n_small, 128, 0, stream>>>(es);
+            }
         }
         if (!el.stats_in_substep)
             k_phase_stats<T, P><<<pl.grid[kKStats], pl.block[kKStats], 0, stream>>>(e, 1);
@@ -2856,7 +2981,7 @@ namespace rbps_gpu
             *blocks_per_sm = a < b ? a : b;
             return rc;
         }
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_substep<T, P>, block, fl_smem);
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_substep<T, P, false>, block, fl_smem);
     }
 
     // Enqueues one step of one large world: 2 + 4 * substeps cooperative
@@ -2902,17 +3027,9 @@ namespace rbps_gpu
     template <class T, class P>
     cudaError_t occupancy_phase(int kernel, int block, int *blocks_per_sm)
     {
-        switch (kernel)
-        {
-        case kKFrame: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_phase_frame<T, P>, block, 0);
-        case kKNarrow: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_phase_narrow<T, P>, block, 0);
-        case kKColor: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_phase_color<T, P>, block, 0);
-        case kKPosition:
-            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_phase_position<T, P>, block, 0);
-        case kKVelocity:
-            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_phase_velocity<T, P>, block, 0);
-        default: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_phase_stats<T, P>, block, 0);
-        }
+        if (kernel == kKFrame)
+            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_phase_frame<T, P>, block, 0);
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_phase_stats<T, P>, block, 0);
     }
 
     template <class T, class P>
@@ -2923,8 +3040,6 @@ namespace rbps_gpu
 } // namespace rbps_gpu
 
 #define RBPS_INSTANTIATE_ENGINE(T, P)                                                                          \
-    template cudaError_t rbps_gpu::launch_step_phases<T, P>(const rbps_gpu::Engine<T, P> &,                        \
-                                                            const rbps_gpu::PhaseLaunch &, cudaStream_t);           \
     template cudaError_t rbps_gpu::launch_step_big<T, P>(const rbps_gpu::Engine<T, P> &, uint32_t, int, int,        \
                                                          cudaStream_t, long *);                                   \
     template cudaError_t rbps_gpu::occupancy_phase<T, P>(int, int, int *);                                         \

@@ -69,7 +69,8 @@ namespace rbps_gpu
         size_t yz;               // float y / z extents per SAP object (float4), grid worlds only
         size_t corder;           // candidates sorted by colour
         size_t misc;             // small counters
-        size_t act, alist;       // active-candidate flags / compacted list (colored mode)
+        size_t act, alist;       // active-candidate flags (then levels) / compacted list
+        size_t lrec, loff;       // reference order: packed bodies of the active candidates, level offsets
         size_t stride;           // bytes per executor
     };
 
@@ -154,6 +155,8 @@ namespace rbps_gpu
         take(L.misc, kMiscWords * 4);
         take(L.act, nc * 4);
         take(L.alist, nc * 4);
+        take(L.lrec, nc * 8);
+        take(L.loff, (nc + 1) * 4);
         L.stride = scr_align(off, 256);
         return L;
     }
@@ -277,16 +280,17 @@ namespace rbps_gpu
 
     // Host entry points, instantiated per precision in engine_f64.cu /
     // engine_f32.cu.  They only enqueue work on `stream`.
-    // Phase kernels of the batched step (one launch per phase).
+    // Phases of a step: the frame and stats phases are kernels of the batched
+    // step; a large world runs all of them, one cooperative launch each.
     enum : int
     {
         kKFrame = 0,
-        kKNarrow = 1,
-        kKColor = 2,
-        kKPosition = 3,
-        kKVelocity = 4,
-        kKStats = 5,
-        kNumPhaseKernels = 6
+        kKStats = 1,
+        kNumPhaseKernels = 2, // with a kernel of their own
+        kKNarrow = 2,
+        kKColor = 3,
+        kKPosition = 4,
+        kKVelocity = 5
     };
     struct PhaseLaunch
     {
@@ -294,10 +298,9 @@ namespace rbps_gpu
         int block[kNumPhaseKernels];
     };
 
-    template <class T, class P>
-    cudaError_t launch_step_phases(const Engine<T, P> &e, const PhaseLaunch &pl, cudaStream_t stream);
-    // Colored mode: the frame / stats phases per world, the substeps flat
-    // over all small worlds (grids: narrowphase, cooperative solves).
+    // The step of the small worlds, in both solve modes: the frame / stats
+    // phases per world, the substeps flat over all small worlds (grids:
+    // narrowphase, cooperative solves).
     struct FlatLaunch
     {
         int grid_narrow, grid_solve, block_solve;
@@ -306,7 +309,7 @@ namespace rbps_gpu
         // a second stream on which the box-box narrowphase runs beside the
         // other classes' (fork / join events), or null for one stream
         cudaStream_t side;
-        cudaEvent_t fork[8], join[8]; // one pair per substep (substeps <= 8), else sequential
+        cudaEvent_t fork, join;
     };
     template <class T, class P>
     cudaError_t launch_step_flat(const Engine<T, P> &e, const PhaseLaunch &pl, const FlatLaunch &fl,
