@@ -1540,6 +1540,14 @@ static int commit_typed(rbps_batch *b)
         CU(cudaEventCreateWithFlags(&b->flat.fork, cudaEventDisableTiming));
         CU(cudaEventCreateWithFlags(&b->flat.join, cudaEventDisableTiming));
     }
+    for (const auto &w : b->worlds)
+        for (const auto &c : w.colliders)
+        {
+            const bool tri = c.shape == RBPS_SHAPE_MESH || c.shape == RBPS_SHAPE_HEIGHTMAP;
+            b->flat.triangles = b->flat.triangles || tri;
+            b->flat.others = b->flat.others || (!tri && c.shape != RBPS_SHAPE_SPHERE && c.shape != RBPS_SHAPE_BOX &&
+                                                c.shape != RBPS_SHAPE_CAPSULE && c.shape != RBPS_SHAPE_PLANE);
+        }
     // ---- GJK pass: only batches with hull colliders reach it
     {
         bool any_hull = false;
@@ -1647,12 +1655,13 @@ static long enqueue_step(rbps_batch *b, const Engine<T, P> &e)
         if (launch_step_flat<T, P>(e, b->phase, b->flat, b->stream) != cudaSuccess)
             return RBPS_ERR_CUDA;
         // frame, prefix, 3 class-sort kernels, stats (only with dumps:
-        // otherwise the last substep writes them); per substep the three
-        // narrowphase kernels, the GJK pass (batches with hulls) and the
+        // otherwise the last substep writes them); per substep the two
+        // narrowphase kernels of the common kinds and those of the kinds the
+        // batch has, the GJK pass (batches with hulls) and the
         // substep (three kernels in float reference order)
         const long solve = e.solve_mode != 1 && sizeof(T) == 4 ? 3 : 1;
         launches += (e.dump_cc || b->desc.substeps < 1 ? 6 : 5) +
-                    (long)b->desc.substeps * (3 + solve + (e.gjk_list ? 1 : 0));
+                    (long)b->desc.substeps * (2 + b->flat.others + b->flat.triangles + solve + (e.gjk_list ? 1 : 0));
     }
     for (uint32_t w : b->big_ids)
     {

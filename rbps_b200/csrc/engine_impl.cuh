@@ -1957,7 +1957,9 @@ namespace rbps_gpu
     //                    warp of the narrowphase runs one pair routine
     // and per substep:
     //   k_flat_narrow    one thread per candidate, in shape-pair order; the
-    //                    box-box class in k_flat_narrow_boxbox
+    //                    box-box class in k_flat_narrow_boxbox, other convex
+    //                    kinds in k_flat_narrow_other, meshes and heightmaps
+    //                    on a warp each in k_flat_narrow_triangles
     //   k_substep        one CTA per large world, one warp per other world:
     //                    greedy colouring of the contacting candidates (in
     //                    reference order their levels), integrate, position
@@ -1991,23 +1993,33 @@ namespace rbps_gpu
             E.wcoff[E.n_small] = carry;
     }
 
-    // Shape-pair class of a candidate, 25 classes over (kind a, kind b) with
-    // the kinds folded to sphere, box, capsule, plane and "other": the 16
-    // pairs of the four common kinds first (ia * 4 + ib; box-box is 5), then
-    // the pairs with an other kind (16-20 other first, 21-24 other second),
-    // so one kernel takes [0, 16) but box-box and another [16, 25).
+    // Shape-pair class of a candidate, over (kind a, kind b) with the kinds
+    // folded to sphere, box, capsule, plane, "other" and "triangles" (mesh,
+    // heightmap): the 16 pairs of the four common kinds first (ia * 4 + ib;
+    // box-box is 5), then the pairs with an other kind (16-20 other first,
+    // 21-24 other second), then those with triangles (25-30 triangles first,
+    // 31-35 second), so one kernel takes [0, 16) but box-box, one [16, 25)
+    // and one [25, 36).
     __device__ __forceinline__ uint32_t kind_index(int kind)
     {
-        return kind == kSphere ? 0u : kind == kBox ? 1u : kind == kCapsule ? 2u : kind == kPlane ? 3u : 4u;
+        return kind == kSphere                           ? 0u
+               : kind == kBox                            ? 1u
+               : kind == kCapsule                        ? 2u
+               : kind == kPlane                          ? 3u
+               : kind == kMesh || kind == kHeightmap     ? 5u
+                                                         : 4u;
     }
     constexpr uint32_t kClassBoxBox = 1u * 4u + 1u; // cand_class of a box-box pair
     constexpr uint32_t kClassCommonEnd = 16u;        // classes [0, 16): common kinds only
+    constexpr uint32_t kClassOtherEnd = 25u;         // classes [25, 36): with triangles
 
     __device__ __forceinline__ uint32_t pair_class(uint32_t ia, uint32_t ib)
     {
         if (ia < 4u && ib < 4u)
             return ia * 4u + ib;
-        return ia == 4u ? 16u + ib : 21u + ia;
+        if (ia < 5u && ib < 5u)
+            return ia == 4u ? 16u + ib : 21u + ia;
+        return ia == 5u ? 25u + ib : 31u + ia;
     }
 
     // The small world holding flat candidate f: last q with wcoff[q] <= f.
@@ -2174,12 +2186,12 @@ namespace rbps_gpu
         }
     }
 
-    // The classes with any other kind (ellipsoid, cylinder, cone, hull,
-    // heightmap, mesh): [off(16), total), with every routine but box-box.
+    // The classes with another convex kind (ellipsoid, cylinder, cone, hull):
+    // [off(16), off(25)).
     template <class T, class P>
     __global__ void __launch_bounds__(kMaxBlock, RBPS_NARROW_MIN_BLOCKS) k_flat_narrow_other(const Engine<T, P> E)
     {
-        const uint32_t o0 = E.gcol[kGcolOff + kClassCommonEnd], total = E.gcol[kGcolOff + kPairClasses];
+        const uint32_t o0 = E.gcol[kGcolOff + kClassCommonEnd], total = E.gcol[kGcolOff + kClassOtherEnd];
         const uint32_t n = total - o0;
         const uint32_t per_warp = E.narrow_per_warp, lane = threadIdx.x & 31u;
         const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -2188,7 +2200,39 @@ namespace rbps_gpu
         {
             const uint32_t end = min(n, base + per_warp);
             for (uint32_t k = base + lane; k < end; k += 32)
-                narrow_flat<T, P, kSelNoBoxBox>(E, o0 + k);
+                narrow_flat<T, P, kSelConvex>(E, o0 + k);
+        }
+    }
+
+    // The classes with a mesh or a heightmap: [off(25), total), a warp a
+    // pair.  A ground mesh's box holds every body of its world, so each pair
+    // runs every face: on one thread the longest such loop was the kernel
+    // (250 shape worlds of 40 bodies, 512-face grounds: 1,235 us a launch;
+    // 62 us with the faces on a warp's lanes).  Consecutive warps
+    // of the list go to different CTAs, so a few pairs spread over the chip.
+    template <class T, class P>
+    __global__ void __launch_bounds__(kMaxBlock) k_flat_narrow_triangles(const Engine<T, P> E)
+    {
+        const uint32_t o0 = E.gcol[kGcolOff + kClassOtherEnd], total = E.gcol[kGcolOff + kPairClasses];
+        const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
+        for (uint32_t i = o0 + (threadIdx.x >> 5) * gridDim.x + blockIdx.x; i < total; i += n_warps)
+        {
+            const uint2 e = E.nlist[i];
+            const uint4 g = E.nglob[i];
+            CandContacts<T, P> &out = E.wcc[e.x][e.y];
+            if (g.x == ~0u) // a corrupt candidate, reported by the class sort
+            {
+                if (lane_id() == 0)
+                    out.n = 0;
+                continue;
+            }
+            const tf<T> ta = collider_tf(E, g.x, g.z);
+            const tf<T> tb = collider_tf(E, g.y, g.w);
+            Manifold<T> m;
+            m.n = 0;
+            const bool hit = dispatch_triangles_warp(E.shape[g.x], ta, E.shape[g.y], tb, E.hulls, m);
+            if (lane_id() == 0)
+                emit_manifold(E, g.x, g.y, g.z, g.w, m, hit ? m.n : 0, out);
         }
     }
 
@@ -2930,23 +2974,19 @@ namespace rbps_gpu
         {
             if (e.gjk_list)
                 cudaMemsetAsync(e.gjk_count, 0, 4, stream);
-            if (fl.side)
             {
-                // the two narrowphase kernels touch disjoint candidates: run
+                // the narrowphase kernels touch disjoint candidates: run
                 // them side by side (a fork / join the graph capture keeps)
                 cudaEventRecord(fl.fork, stream);
                 cudaStreamWaitEvent(fl.side, fl.fork, 0);
                 k_flat_narrow_boxbox<T, P><<<fl.grid_narrow, kMaxBlock, 0, fl.side>>>(e);
-                k_flat_narrow_other<T, P><<<fl.grid_narrow, kMaxBlock, 0, fl.side>>>(e);
+                if (fl.others)
+                    k_flat_narrow_other<T, P><<<fl.grid_narrow, kMaxBlock, 0, fl.side>>>(e);
+                if (fl.triangles)
+                    k_flat_narrow_triangles<T, P><<<fl.grid_narrow, kMaxBlock, 0, fl.side>>>(e);
                 cudaEventRecord(fl.join, fl.side);
                 k_flat_narrow<T, P><<<fl.grid_narrow, kMaxBlock, 0, stream>>>(e);
                 cudaStreamWaitEvent(stream, fl.join, 0);
-            }
-            else
-            {
-                k_flat_narrow<T, P><<<fl.grid_narrow, kMaxBlock, 0, stream>>>(e);
-                k_flat_narrow_boxbox<T, P><<<fl.grid_narrow, kMaxBlock, 0, stream>>>(e);
-                k_flat_narrow_other<T, P><<<fl.grid_narrow, kMaxBlock, 0, stream>>>(e);
             }
             launch_gjk(e, stream);
             const Engine<T, P> &es = s + 1 == e.substeps ? el : e;

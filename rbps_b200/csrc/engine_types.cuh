@@ -273,10 +273,10 @@ namespace rbps_gpu
         uint32_t n_sjcolors, n_sjoints;
     };
 
-    // gcol layout (u32 words): per shape-pair class [0, 32) counts, [32, 64)
-    // fill cursors, [64, 96) offsets (entry kPairClasses = total)
-    constexpr uint32_t kPairClasses = 25;
-    constexpr uint32_t kGcolCount = 0, kGcolFill = 32, kGcolOff = 64, kGcolWords = 96;
+    // gcol layout (u32 words): per shape-pair class [0, 64) counts, [64, 128)
+    // fill cursors, [128, 192) offsets (entry kPairClasses = total)
+    constexpr uint32_t kPairClasses = 36;
+    constexpr uint32_t kGcolCount = 0, kGcolFill = 64, kGcolOff = 128, kGcolWords = 192;
 
     // Host entry points, instantiated per precision in engine_f64.cu /
     // engine_f32.cu.  They only enqueue work on `stream`.
@@ -306,6 +306,7 @@ namespace rbps_gpu
         int grid_narrow, grid_solve, block_solve;
         int grid_sort;       // the class-sort kernels: every CTA they can keep resident
         size_t substep_smem; // dynamic shared memory of k_substep
+        bool triangles, others; // the batch has meshes or heightmaps / other kinds beyond sphere, box, capsule, plane
         // a second stream on which the box-box narrowphase runs beside the
         // other classes' (fork / join events), or null for one stream
         cudaStream_t side;

@@ -1326,21 +1326,69 @@ namespace rbps_gpu
         return true;
     }
 
+    // The triangle loops below (a mesh's faces, the cells of a heightmap)
+    // keep the first deepest contact.  With Lanes == 32 a warp runs one pair:
+    // lane l takes every 32nd face (or cell) from l, and this leaves the
+    // pair's contact, that of the lowest face `at` among the deepest, on
+    // every lane.  Per face the arithmetic is the same, so the result is too.
+    template <class T, int Lanes>
+    __device__ __forceinline__ bool deepest_of_lanes(bool hit, T best, uint32_t at, Manifold<T> &out)
+    {
+        if constexpr (Lanes == 32)
+        {
+            if (!hit)
+                at = ~0u;
+            for (int o = 16; o; o >>= 1)
+            {
+                const T d = __shfl_xor_sync(0xffffffffu, best, o);
+                const uint32_t k = __shfl_xor_sync(0xffffffffu, at, o);
+                if (k != ~0u && (at == ~0u || d > best || (d == best && k < at)))
+                {
+                    best = d;
+                    at = k;
+                }
+            }
+            if (at == ~0u)
+                return false;
+            const int src = (int)(at & 31u); // face t is lane t % 32's
+            out.n = 1;
+            out.depth[0] = best;
+            out.normal = vec3<T>(__shfl_sync(0xffffffffu, out.normal.x, src), __shfl_sync(0xffffffffu, out.normal.y, src),
+                                 __shfl_sync(0xffffffffu, out.normal.z, src));
+            out.pos[0] = vec3<T>(__shfl_sync(0xffffffffu, out.pos[0].x, src), __shfl_sync(0xffffffffu, out.pos[0].y, src),
+                                 __shfl_sync(0xffffffffu, out.pos[0].z, src));
+            return true;
+        }
+        return hit;
+    }
+
     // heightmap_test (HeightmapCollision.hpp): shape `kind` (see
-    // tri_contact) with world AABB [qmn, qmx] against heightmap `id`.
+    // tri_contact) with world AABB [qmn, qmx] against the cells of heightmap
+    // `id` under it: all of them, or, with `cells`, the one of that index in
+    // row order (*cells receives their count).  Out of line, so that float
+    // contracts the same way in every caller.
     template <class T>
-    __device__ bool heightmap_contact(const HullSetDev &hs, uint32_t id, int kind, const vec3<T> &p0,
+    __device__ __noinline__ bool heightmap_cells(const HullSetDev &hs, uint32_t id, int kind, const vec3<T> &p0,
                                       const vec3<T> &p1, T r, const tf<T> &tb, const vec3<T> &h,
-                                      const vec3<T> &qmn, const vec3<T> &qmx, Manifold<T> &out)
+                                      const vec3<T> &qmn, const vec3<T> &qmx, Manifold<T> &out, uint32_t cell, uint32_t *cells)
     {
         const HmDesc &hd = hs.hm_desc[id];
         const float *H = hs.hm_heights + hd.off;
         const T ox = T(hd.origin[0]), oy = T(hd.origin[1]), oz = T(hd.origin[2]);
         const T sx = T(hd.scale[0]), sy = T(hd.scale[1]), sz = T(hd.scale[2]);
-        const int r0 = max(0, int((qmn.z - oz) / sz));
-        const int r1 = min(int(hd.rows) - 2, int((qmx.z - oz) / sz));
-        const int c0 = max(0, int((qmn.x - ox) / sx));
-        const int c1 = min(int(hd.cols) - 2, int((qmx.x - ox) / sx));
+        int r0 = max(0, int((qmn.z - oz) / sz));
+        int r1 = min(int(hd.rows) - 2, int((qmx.z - oz) / sz));
+        int c0 = max(0, int((qmn.x - ox) / sx));
+        int c1 = min(int(hd.cols) - 2, int((qmx.x - ox) / sx));
+        if (cells) // this cell of them alone
+        {
+            const uint32_t nc = c1 >= c0 ? uint32_t(c1 - c0 + 1) : 0u;
+            *cells = r1 >= r0 ? nc * uint32_t(r1 - r0 + 1) : 0u;
+            if (cell >= *cells)
+                return false;
+            r0 = r1 = r0 + int(cell / nc);
+            c0 = c1 = c0 + int(cell % nc);
+        }
         auto vtx = [&](int row, int col) {
             return vec3<T>(ox + T(col) * sx, T(H[(uint32_t)row * hd.cols + (uint32_t)col]) * sy + oy, oz + T(row) * sz);
         };
@@ -1367,10 +1415,37 @@ namespace rbps_gpu
         return hit;
     }
 
+
+    // heightmap_cells on one thread, or a cell at a time on a warp's lanes.
+    template <class T, int Lanes>
+    __device__ bool heightmap_contact(const HullSetDev &hs, uint32_t id, int kind, const vec3<T> &p0,
+                                      const vec3<T> &p1, T r, const tf<T> &tb, const vec3<T> &h,
+                                      const vec3<T> &qmn, const vec3<T> &qmx, Manifold<T> &out)
+    {
+        if constexpr (Lanes == 1)
+            return heightmap_cells(hs, id, kind, p0, p1, r, tb, h, qmn, qmx, out, 0, nullptr);
+        bool hit = false;
+        T best = T(0.0);
+        uint32_t at = 0, cells = ~0u;
+        for (uint32_t cell = threadIdx.x & 31u; cell < cells; cell += 32u)
+        {
+            Manifold<T> cand;
+            cand.n = 0;
+            if (heightmap_cells(hs, id, kind, p0, p1, r, tb, h, qmn, qmx, cand, cell, &cells) && cand.depth[0] > best)
+            {
+                best = cand.depth[0];
+                out = cand;
+                at = cell;
+                hit = true;
+            }
+        }
+        return deepest_of_lanes<T, Lanes>(hit, best, at, out);
+    }
+
     // Sphere / Capsule / Box (shape a) against heightmap hm; other shapes
     // against a heightmap find no contact (the primary CollisionAlgorithm of
     // a non-convex pair, Dispatcher.hpp:40-60).
-    template <class T>
+    template <class T, int Lanes = 1>
     __device__ bool shape_heightmap(const ShapeDev &sa, const tf<T> &ta, const ShapeDev &hm, const HullSetDev &hs,
                                     Manifold<T> &m)
     {
@@ -1379,7 +1454,7 @@ namespace rbps_gpu
         {
             const T r = T(sa.p[0]);
             const vec3<T> rr(r, r, r);
-            return heightmap_contact(hs, uint32_t(hm.hull), 0, ta.pos, zero, r, ta, zero, ta.pos - rr, ta.pos + rr, m);
+            return heightmap_contact<T, Lanes>(hs, uint32_t(hm.hull), 0, ta.pos, zero, r, ta, zero, ta.pos - rr, ta.pos + rr, m);
         }
         if (sa.kind == kCapsule) // capsule_endpoints + compute_aabb(Capsule)
         {
@@ -1391,7 +1466,7 @@ namespace rbps_gpu
             const vec3<T> rr(r, r, r);
             const vec3<T> qmn = vec3<T>(rmin(a1.x, a2.x), rmin(a1.y, a2.y), rmin(a1.z, a2.z)) - rr;
             const vec3<T> qmx = vec3<T>(rmax(a1.x, a2.x), rmax(a1.y, a2.y), rmax(a1.z, a2.z)) + rr;
-            return heightmap_contact(hs, uint32_t(hm.hull), 1, p1, p2, r, ta, zero, qmn, qmx, m);
+            return heightmap_contact<T, Lanes>(hs, uint32_t(hm.hull), 1, p1, p2, r, ta, zero, qmn, qmx, m);
         }
         if (sa.kind == kBox) // compute_aabb(Box)
         {
@@ -1400,7 +1475,7 @@ namespace rbps_gpu
             const vec3<T> e(rabs(R.c[0].x) * h.x + rabs(R.c[1].x) * h.y + rabs(R.c[2].x) * h.z,
                             rabs(R.c[0].y) * h.x + rabs(R.c[1].y) * h.y + rabs(R.c[2].y) * h.z,
                             rabs(R.c[0].z) * h.x + rabs(R.c[1].z) * h.y + rabs(R.c[2].z) * h.z);
-            return heightmap_contact(hs, uint32_t(hm.hull), 2, zero, zero, T(0), ta, h, ta.pos - e, ta.pos + e, m);
+            return heightmap_contact<T, Lanes>(hs, uint32_t(hm.hull), 2, zero, zero, T(0), ta, h, ta.pos - e, ta.pos + e, m);
         }
         return false;
     }
@@ -1427,14 +1502,15 @@ namespace rbps_gpu
     // mesh_test_all with the sphere / capsule / box per-triangle tests
     // (kind 0 / 1 / 2; the box test is the mesh's own: depth = box_r -
     // edge distance, kept when positive), deepest contact of all faces.
-    template <class T>
+    template <class T, int Lanes>
     __device__ bool mesh_contact(const HullSetDev &hs, uint32_t id, const tf<T> &tm, int kind, const vec3<T> &p0,
                                  const vec3<T> &p1, T r, const tf<T> &tb, const vec3<T> &h, Manifold<T> &out)
     {
         const MeshDesc &md = hs.mesh[id];
         bool hit = false;
         T best = T(0.0);
-        for (uint32_t f = 0; f < md.nf; ++f)
+        uint32_t at = 0;
+        for (uint32_t f = Lanes == 32 ? threadIdx.x & 31u : 0u; f < md.nf; f += Lanes)
         {
             vec3<T> A, B, C, n;
             mesh_triangle(hs, md, f, tm, A, B, C, n);
@@ -1468,15 +1544,16 @@ namespace rbps_gpu
             {
                 best = cand.depth[0];
                 out = cand;
+                at = f;
                 hit = true;
             }
         }
-        return hit;
+        return deepest_of_lanes<T, Lanes>(hit, best, at, out);
     }
 
     // Mesh vs Mesh (MeshCollision.hpp): every vertex of every face of A as a
     // sphere of radius 0 against all faces of B, the deepest kept.
-    template <class T>
+    template <class T, int Lanes>
     __device__ bool mesh_mesh(const HullSetDev &hs, uint32_t ia, const tf<T> &ta, uint32_t ib, const tf<T> &tb,
                               Manifold<T> &out)
     {
@@ -1492,7 +1569,7 @@ namespace rbps_gpu
             mesh_triangle(hs, ma, f, ta, A, B, C, n);
             const vec3<T> verts[3] = {A, B, C};
             for (int k = 0; k < 3; ++k)
-                if (mesh_contact(hs, ib, tb, 0, verts[k], zero, T(0.0), tb, zero, cand) && cand.depth[0] > best)
+                if (mesh_contact<T, Lanes>(hs, ib, tb, 0, verts[k], zero, T(0.0), tb, zero, cand) && cand.depth[0] > best)
                 {
                     best = cand.depth[0];
                     out = cand;
@@ -1504,30 +1581,30 @@ namespace rbps_gpu
 
     // Sphere / Capsule / Box (shape a) or a mesh against mesh `mesh`; other
     // shapes find no contact (the primary algorithm of a non-convex pair).
-    template <class T>
+    template <class T, int Lanes = 1>
     __device__ bool shape_mesh(const ShapeDev &sa, const tf<T> &ta, const ShapeDev &mesh, const tf<T> &tm,
                                const HullSetDev &hs, Manifold<T> &m)
     {
         const vec3<T> zero(T(0), T(0), T(0));
         const uint32_t id = uint32_t(mesh.hull);
         if (sa.kind == kSphere)
-            return mesh_contact(hs, id, tm, 0, ta.pos, zero, T(sa.p[0]), ta, zero, m);
+            return mesh_contact<T, Lanes>(hs, id, tm, 0, ta.pos, zero, T(sa.p[0]), ta, zero, m);
         if (sa.kind == kCapsule)
         {
             vec3<T> p1, p2;
             capsule_endpoints(T(sa.p[0]), ta, p1, p2);
-            return mesh_contact(hs, id, tm, 1, p1, p2, T(sa.p[1]), ta, zero, m);
+            return mesh_contact<T, Lanes>(hs, id, tm, 1, p1, p2, T(sa.p[1]), ta, zero, m);
         }
         if (sa.kind == kBox)
-            return mesh_contact(hs, id, tm, 2, zero, zero, T(0), ta, vec3<T>(T(sa.p[0]), T(sa.p[1]), T(sa.p[2])), m);
+            return mesh_contact<T, Lanes>(hs, id, tm, 2, zero, zero, T(0), ta, vec3<T>(T(sa.p[0]), T(sa.p[1]), T(sa.p[2])), m);
         if (sa.kind == kMesh)
-            return mesh_mesh(hs, uint32_t(sa.hull), ta, id, tm, m);
+            return mesh_mesh<T, Lanes>(hs, uint32_t(sa.hull), ta, id, tm, m);
         return false;
     }
 
     // convex_vs_plane for a mesh (RBC_PLANE_SPEC(Mesh)): the support vertex
     // along -n (first of the largest dot products, Mesh.hpp support).
-    template <class T>
+    template <class T, int Lanes = 1>
     __device__ bool mesh_plane(const HullSetDev &hs, uint32_t id, const tf<T> &ts, const ShapeDev &pl, const tf<T> &tp,
                                Manifold<T> &out)
     {
@@ -1540,9 +1617,13 @@ namespace rbps_gpu
         if (md.nv)
         {
             const double *V = hs.mesh_v + 3 * (size_t)md.v0;
+            // lane 0 starts from vertex 0 as the serial scan does, the
+            // others of a warp from none
+            const uint32_t lane = Lanes == 32 ? threadIdx.x & 31u : 0u;
             ls = vec3<T>(T(V[0]), T(V[1]), T(V[2]));
-            T bd = dot(ls, ld);
-            for (uint32_t i = 1; i < md.nv; ++i)
+            T bd = lane ? -T(HUGE_VAL) : dot(ls, ld);
+            uint32_t at = lane ? ~0u : 0u;
+            for (uint32_t i = lane ? lane : Lanes; i < md.nv; i += Lanes)
             {
                 const vec3<T> p{T(V[3 * i]), T(V[3 * i + 1]), T(V[3 * i + 2])};
                 const T d = dot(p, ld);
@@ -1550,7 +1631,23 @@ namespace rbps_gpu
                 {
                     bd = d;
                     ls = p;
+                    at = i;
                 }
+            }
+            if constexpr (Lanes == 32)
+            {
+                for (int o = 16; o; o >>= 1)
+                {
+                    const T d = __shfl_xor_sync(0xffffffffu, bd, o);
+                    const uint32_t k = __shfl_xor_sync(0xffffffffu, at, o);
+                    if (k != ~0u && (d > bd || (d == bd && k < at)))
+                    {
+                        bd = d;
+                        at = k;
+                    }
+                }
+                at = __shfl_sync(0xffffffffu, at, 0);
+                ls = vec3<T>(T(V[3 * at]), T(V[3 * at + 1]), T(V[3 * at + 2]));
             }
         }
         const vec3<T> ws = ts.pos + ts.rotate_vector(ls);
@@ -1564,12 +1661,13 @@ namespace rbps_gpu
         return true;
     }
 
-    // Sel selects the routines compiled in: kSelAll every pair; kSelNoBoxBox
-    // all but box-box; kSelBoxBox box-box only; kSelCommon the pairs of
-    // spheres, boxes, capsules and planes but box-box (the caller guarantees
-    // the kinds), so a kernel carries only the code, registers and local
-    // buffers of the routines it can meet.
-    constexpr int kSelAll = 0, kSelNoBoxBox = 1, kSelBoxBox = 2, kSelCommon = 3;
+    // Sel selects the routines compiled in: kSelAll every pair; kSelConvex
+    // those with an ellipsoid, cylinder, cone or hull but no triangles;
+    // kSelBoxBox box-box only; kSelCommon the pairs of spheres, boxes,
+    // capsules and planes but box-box (the caller guarantees the kinds), so
+    // a kernel carries only the code, registers and local buffers of the
+    // routines it can meet.
+    constexpr int kSelAll = 0, kSelConvex = 1, kSelBoxBox = 2, kSelCommon = 3;
 
     template <class T, int Sel = kSelAll>
     __device__ __forceinline__ int dispatch_pair(const ShapeDev &sa, const tf<T> &ta, const ShapeDev &sb,
@@ -1581,6 +1679,7 @@ namespace rbps_gpu
                        ? kHit
                        : kMiss;
         constexpr bool kAny = Sel != kSelCommon; // kinds beyond the four common ones
+        constexpr bool kTri = Sel == kSelAll;    // meshes and heightmaps
         const int ka = sa.kind, kb = sb.kind;
         bool hit = false;
         bool flip = false;
@@ -1602,7 +1701,7 @@ namespace rbps_gpu
                 hit = cylinder_plane(T(sa.p[0]), T(sa.p[1]), ta, sb, tb, m);
             else if (ka == kEllipsoid || ka == kCone)
                 hit = round_plane(sa, ta, sb, tb, m);
-            else if (ka == kMesh)
+            else if (kTri && ka == kMesh)
                 hit = mesh_plane(hs, uint32_t(sa.hull), ta, sb, tb, m);
             return hit ? kHit : kMiss;
         }
@@ -1624,13 +1723,13 @@ namespace rbps_gpu
                 hit = cylinder_plane(T(sb.p[0]), T(sb.p[1]), tb, sa, ta, m);
             else if (kb == kEllipsoid || kb == kCone)
                 hit = round_plane(sb, tb, sa, ta, m);
-            else if (kb == kMesh)
+            else if (kTri && kb == kMesh)
                 hit = mesh_plane(hs, uint32_t(sb.hull), tb, sa, ta, m);
             if (hit)
                 m.normal = -m.normal;
             return hit ? kHit : kMiss;
         }
-        if (kAny && (ka == kMesh || kb == kMesh))
+        if (kTri && (ka == kMesh || kb == kMesh))
         {
             if (ka == kHeightmap || kb == kHeightmap)
                 return kMiss; // no Mesh / Heightmap algorithm: the primary one finds nothing
@@ -1644,7 +1743,7 @@ namespace rbps_gpu
             }
             return hit ? kHit : kMiss;
         }
-        if (kAny && (ka == kHeightmap || kb == kHeightmap))
+        if (kTri && (ka == kHeightmap || kb == kHeightmap))
         {
             if (kb == kHeightmap)
                 hit = shape_heightmap(sa, ta, sb, hs, m);
@@ -1658,6 +1757,8 @@ namespace rbps_gpu
         }
         if (kAny && (gjk_kind(ka) || gjk_kind(kb)))
             return kNeedsGjk;
+        if (Sel == kSelConvex)
+            return kMiss; // the caller's classes all have such a kind
         if (ka == kSphere && kb == kSphere)
             hit = sphere_sphere(T(sa.p[0]), ta, T(sb.p[0]), tb, m);
         else if (ka == kSphere && kb == kBox)
@@ -1688,5 +1789,37 @@ namespace rbps_gpu
         if (hit && flip)
             m.normal = -m.normal;
         return hit ? kHit : kMiss;
+    }
+
+    // A pair with a mesh or a heightmap on one warp: dispatch_pair's routines
+    // for those kinds with their triangle loops split over the lanes.  Every
+    // lane holds the result.
+    template <class T>
+    __device__ __forceinline__ bool dispatch_triangles_warp(const ShapeDev &sa, const tf<T> &ta, const ShapeDev &sb,
+                                                            const tf<T> &tb, const HullSetDev &hs, Manifold<T> &m)
+    {
+        bool hit = false, flip = false;
+        if (sb.kind == kPlane)
+            hit = sa.kind == kMesh && mesh_plane<T, 32>(hs, uint32_t(sa.hull), ta, sb, tb, m);
+        else if (sa.kind == kPlane)
+        {
+            hit = sb.kind == kMesh && mesh_plane<T, 32>(hs, uint32_t(sb.hull), tb, sa, ta, m);
+            flip = true;
+        }
+        else if (sa.kind == kMesh || sb.kind == kMesh)
+        {
+            if (sa.kind == kHeightmap || sb.kind == kHeightmap)
+                return false; // no Mesh / Heightmap algorithm: the primary one finds nothing
+            flip = sb.kind != kMesh; // CollisionAlgorithmSym
+            hit = flip ? shape_mesh<T, 32>(sb, tb, sa, ta, hs, m) : shape_mesh<T, 32>(sa, ta, sb, tb, hs, m);
+        }
+        else
+        {
+            flip = sb.kind != kHeightmap;
+            hit = flip ? shape_heightmap<T, 32>(sb, tb, sa, hs, m) : shape_heightmap<T, 32>(sa, ta, sb, hs, m);
+        }
+        if (hit && flip)
+            m.normal = -m.normal;
+        return hit;
     }
 } // namespace rbps_gpu
