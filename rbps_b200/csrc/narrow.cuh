@@ -1362,13 +1362,12 @@ namespace rbps_gpu
         return hit;
     }
 
-    // heightmap_test (HeightmapCollision.hpp): shape `kind` (see
-    // tri_contact) with world AABB [qmn, qmx] against the cells of heightmap
-    // `id` under it: all of them, or, with `cells`, the one of that index in
-    // row order (*cells receives their count).  Out of line, so that float
-    // contracts the same way in every caller.
+    // heightmap_contact's test of one cell under the shape, the one of index
+    // `cell` in row order; *cells receives their count.  Out of line, and
+    // beside the serial form rather than under it: float contracts into FMAs
+    // by function, and the results are to be those of the serial loops.
     template <class T>
-    __device__ __noinline__ bool heightmap_cells(const HullSetDev &hs, uint32_t id, int kind, const vec3<T> &p0,
+    __device__ __noinline__ bool heightmap_cell(const HullSetDev &hs, uint32_t id, int kind, const vec3<T> &p0,
                                       const vec3<T> &p1, T r, const tf<T> &tb, const vec3<T> &h,
                                       const vec3<T> &qmn, const vec3<T> &qmx, Manifold<T> &out, uint32_t cell, uint32_t *cells)
     {
@@ -1380,7 +1379,6 @@ namespace rbps_gpu
         int r1 = min(int(hd.rows) - 2, int((qmx.z - oz) / sz));
         int c0 = max(0, int((qmn.x - ox) / sx));
         int c1 = min(int(hd.cols) - 2, int((qmx.x - ox) / sx));
-        if (cells) // this cell of them alone
         {
             const uint32_t nc = c1 >= c0 ? uint32_t(c1 - c0 + 1) : 0u;
             *cells = r1 >= r0 ? nc * uint32_t(r1 - r0 + 1) : 0u;
@@ -1415,15 +1413,12 @@ namespace rbps_gpu
         return hit;
     }
 
-
-    // heightmap_cells on one thread, or a cell at a time on a warp's lanes.
-    template <class T, int Lanes>
-    __device__ bool heightmap_contact(const HullSetDev &hs, uint32_t id, int kind, const vec3<T> &p0,
+    // heightmap_contact on a warp, a cell at a time on each lane.
+    template <class T>
+    __device__ bool heightmap_contact_warp(const HullSetDev &hs, uint32_t id, int kind, const vec3<T> &p0,
                                       const vec3<T> &p1, T r, const tf<T> &tb, const vec3<T> &h,
                                       const vec3<T> &qmn, const vec3<T> &qmx, Manifold<T> &out)
     {
-        if constexpr (Lanes == 1)
-            return heightmap_cells(hs, id, kind, p0, p1, r, tb, h, qmn, qmx, out, 0, nullptr);
         bool hit = false;
         T best = T(0.0);
         uint32_t at = 0, cells = ~0u;
@@ -1431,7 +1426,7 @@ namespace rbps_gpu
         {
             Manifold<T> cand;
             cand.n = 0;
-            if (heightmap_cells(hs, id, kind, p0, p1, r, tb, h, qmn, qmx, cand, cell, &cells) && cand.depth[0] > best)
+            if (heightmap_cell(hs, id, kind, p0, p1, r, tb, h, qmn, qmx, cand, cell, &cells) && cand.depth[0] > best)
             {
                 best = cand.depth[0];
                 out = cand;
@@ -1439,14 +1434,14 @@ namespace rbps_gpu
                 hit = true;
             }
         }
-        return deepest_of_lanes<T, Lanes>(hit, best, at, out);
+        return deepest_of_lanes<T, 32>(hit, best, at, out);
     }
 
     // Sphere / Capsule / Box (shape a) against heightmap hm; other shapes
     // against a heightmap find no contact (the primary CollisionAlgorithm of
     // a non-convex pair, Dispatcher.hpp:40-60).
-    template <class T, int Lanes = 1>
-    __device__ bool shape_heightmap(const ShapeDev &sa, const tf<T> &ta, const ShapeDev &hm, const HullSetDev &hs,
+    template <class T>
+    __device__ bool shape_heightmap_warp(const ShapeDev &sa, const tf<T> &ta, const ShapeDev &hm, const HullSetDev &hs,
                                     Manifold<T> &m)
     {
         const vec3<T> zero(T(0), T(0), T(0));
@@ -1454,7 +1449,7 @@ namespace rbps_gpu
         {
             const T r = T(sa.p[0]);
             const vec3<T> rr(r, r, r);
-            return heightmap_contact<T, Lanes>(hs, uint32_t(hm.hull), 0, ta.pos, zero, r, ta, zero, ta.pos - rr, ta.pos + rr, m);
+            return heightmap_contact_warp(hs, uint32_t(hm.hull), 0, ta.pos, zero, r, ta, zero, ta.pos - rr, ta.pos + rr, m);
         }
         if (sa.kind == kCapsule) // capsule_endpoints + compute_aabb(Capsule)
         {
@@ -1466,7 +1461,7 @@ namespace rbps_gpu
             const vec3<T> rr(r, r, r);
             const vec3<T> qmn = vec3<T>(rmin(a1.x, a2.x), rmin(a1.y, a2.y), rmin(a1.z, a2.z)) - rr;
             const vec3<T> qmx = vec3<T>(rmax(a1.x, a2.x), rmax(a1.y, a2.y), rmax(a1.z, a2.z)) + rr;
-            return heightmap_contact<T, Lanes>(hs, uint32_t(hm.hull), 1, p1, p2, r, ta, zero, qmn, qmx, m);
+            return heightmap_contact_warp(hs, uint32_t(hm.hull), 1, p1, p2, r, ta, zero, qmn, qmx, m);
         }
         if (sa.kind == kBox) // compute_aabb(Box)
         {
@@ -1475,7 +1470,86 @@ namespace rbps_gpu
             const vec3<T> e(rabs(R.c[0].x) * h.x + rabs(R.c[1].x) * h.y + rabs(R.c[2].x) * h.z,
                             rabs(R.c[0].y) * h.x + rabs(R.c[1].y) * h.y + rabs(R.c[2].y) * h.z,
                             rabs(R.c[0].z) * h.x + rabs(R.c[1].z) * h.y + rabs(R.c[2].z) * h.z);
-            return heightmap_contact<T, Lanes>(hs, uint32_t(hm.hull), 2, zero, zero, T(0), ta, h, ta.pos - e, ta.pos + e, m);
+            return heightmap_contact_warp(hs, uint32_t(hm.hull), 2, zero, zero, T(0), ta, h, ta.pos - e, ta.pos + e, m);
+        }
+        return false;
+    }
+
+    // heightmap_test (HeightmapCollision.hpp): shape `kind` (see
+    // tri_contact) with world AABB [qmn, qmx] against heightmap `id`.
+    template <class T>
+    __device__ bool heightmap_contact(const HullSetDev &hs, uint32_t id, int kind, const vec3<T> &p0,
+                                      const vec3<T> &p1, T r, const tf<T> &tb, const vec3<T> &h,
+                                      const vec3<T> &qmn, const vec3<T> &qmx, Manifold<T> &out)
+    {
+        const HmDesc &hd = hs.hm_desc[id];
+        const float *H = hs.hm_heights + hd.off;
+        const T ox = T(hd.origin[0]), oy = T(hd.origin[1]), oz = T(hd.origin[2]);
+        const T sx = T(hd.scale[0]), sy = T(hd.scale[1]), sz = T(hd.scale[2]);
+        const int r0 = max(0, int((qmn.z - oz) / sz));
+        const int r1 = min(int(hd.rows) - 2, int((qmx.z - oz) / sz));
+        const int c0 = max(0, int((qmn.x - ox) / sx));
+        const int c1 = min(int(hd.cols) - 2, int((qmx.x - ox) / sx));
+        auto vtx = [&](int row, int col) {
+            return vec3<T>(ox + T(col) * sx, T(H[(uint32_t)row * hd.cols + (uint32_t)col]) * sy + oy, oz + T(row) * sz);
+        };
+        bool hit = false;
+        T best = T(0.0);
+        for (int rr = r0; rr <= r1; ++rr)
+            for (int cc = c0; cc <= c1; ++cc)
+            {
+                const vec3<T> V00 = vtx(rr, cc), V10 = vtx(rr + 1, cc), V01 = vtx(rr, cc + 1), V11 = vtx(rr + 1, cc + 1);
+                for (int k = 0; k < 2; ++k)
+                {
+                    const vec3<T> A = k ? V10 : V00, B = k ? V11 : V10, C = V01;
+                    const vec3<T> n = normalize(cross(B - A, C - A));
+                    Manifold<T> cand;
+                    cand.n = 0;
+                    if (tri_contact(kind, p0, p1, r, tb, h, A, B, C, n, cand) && cand.depth[0] > best)
+                    {
+                        best = cand.depth[0];
+                        out = cand;
+                        hit = true;
+                    }
+                }
+            }
+        return hit;
+    }
+
+    // Sphere / Capsule / Box (shape a) against heightmap hm; other shapes
+    // against a heightmap find no contact (the primary CollisionAlgorithm of
+    // a non-convex pair, Dispatcher.hpp:40-60).
+    template <class T>
+    __device__ bool shape_heightmap(const ShapeDev &sa, const tf<T> &ta, const ShapeDev &hm, const HullSetDev &hs,
+                                    Manifold<T> &m)
+    {
+        const vec3<T> zero(T(0), T(0), T(0));
+        if (sa.kind == kSphere) // compute_aabb(Sphere)
+        {
+            const T r = T(sa.p[0]);
+            const vec3<T> rr(r, r, r);
+            return heightmap_contact(hs, uint32_t(hm.hull), 0, ta.pos, zero, r, ta, zero, ta.pos - rr, ta.pos + rr, m);
+        }
+        if (sa.kind == kCapsule) // capsule_endpoints + compute_aabb(Capsule)
+        {
+            const T hh = T(sa.p[0]), r = T(sa.p[1]);
+            vec3<T> p1, p2;
+            capsule_endpoints(hh, ta, p1, p2);
+            const vec3<T> axis = ta.rotate_vector(vec3<T>(T(0.0), hh, T(0.0)));
+            const vec3<T> a1 = ta.pos + axis, a2 = ta.pos - axis;
+            const vec3<T> rr(r, r, r);
+            const vec3<T> qmn = vec3<T>(rmin(a1.x, a2.x), rmin(a1.y, a2.y), rmin(a1.z, a2.z)) - rr;
+            const vec3<T> qmx = vec3<T>(rmax(a1.x, a2.x), rmax(a1.y, a2.y), rmax(a1.z, a2.z)) + rr;
+            return heightmap_contact(hs, uint32_t(hm.hull), 1, p1, p2, r, ta, zero, qmn, qmx, m);
+        }
+        if (sa.kind == kBox) // compute_aabb(Box)
+        {
+            const vec3<T> h(T(sa.p[0]), T(sa.p[1]), T(sa.p[2]));
+            const mat3<T> R = mat3_cast(ta.rot);
+            const vec3<T> e(rabs(R.c[0].x) * h.x + rabs(R.c[1].x) * h.y + rabs(R.c[2].x) * h.z,
+                            rabs(R.c[0].y) * h.x + rabs(R.c[1].y) * h.y + rabs(R.c[2].y) * h.z,
+                            rabs(R.c[0].z) * h.x + rabs(R.c[1].z) * h.y + rabs(R.c[2].z) * h.z);
+            return heightmap_contact(hs, uint32_t(hm.hull), 2, zero, zero, T(0), ta, h, ta.pos - e, ta.pos + e, m);
         }
         return false;
     }
@@ -1816,7 +1890,7 @@ namespace rbps_gpu
         else
         {
             flip = sb.kind != kHeightmap;
-            hit = flip ? shape_heightmap<T, 32>(sb, tb, sa, hs, m) : shape_heightmap<T, 32>(sa, ta, sb, hs, m);
+            hit = flip ? shape_heightmap_warp(sb, tb, sa, hs, m) : shape_heightmap_warp(sa, ta, sb, hs, m);
         }
         if (hit && flip)
             m.normal = -m.normal;
