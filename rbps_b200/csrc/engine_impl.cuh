@@ -2973,22 +2973,23 @@ namespace rbps_gpu
         for (int s = 0; s < e.substeps; ++s)
         {
             if (e.gjk_list)
-                cudaMemsetAsync(e.gjk_count, 0, 4, stream);
-            {
-                // the narrowphase kernels touch disjoint candidates: run
-                // them side by side (a fork / join the graph capture keeps)
-                cudaEventRecord(fl.fork, stream);
-                cudaStreamWaitEvent(fl.side, fl.fork, 0);
-                k_flat_narrow_boxbox<T, P><<<fl.grid_narrow, kMaxBlock, 0, fl.side>>>(e);
-                if (fl.others)
-                    k_flat_narrow_other<T, P><<<fl.grid_narrow, kMaxBlock, 0, fl.side>>>(e);
-                if (fl.triangles)
-                    k_flat_narrow_triangles<T, P><<<fl.grid_narrow, kMaxBlock, 0, fl.side>>>(e);
-                cudaEventRecord(fl.join, fl.side);
-                k_flat_narrow<T, P><<<fl.grid_narrow, kMaxBlock, 0, stream>>>(e);
-                cudaStreamWaitEvent(stream, fl.join, 0);
-            }
+                cudaMemsetAsync(e.gjk_count, 0, 8, stream);
+            // the narrowphase kernels touch disjoint candidates: run them
+            // side by side (a fork / join the graph capture keeps).  Only the
+            // other kinds' kernel queues GJK pairs, and the GJK pass is the
+            // longest of all (its few slow pairs, not their number): those
+            // two go first and the rest beside them
+            cudaEventRecord(fl.fork, stream);
+            cudaStreamWaitEvent(fl.side, fl.fork, 0);
+            k_flat_narrow_boxbox<T, P><<<fl.grid_narrow, kMaxBlock, 0, fl.side>>>(e);
+            if (fl.triangles)
+                k_flat_narrow_triangles<T, P><<<fl.grid_narrow, kMaxBlock, 0, fl.side>>>(e);
+            k_flat_narrow<T, P><<<fl.grid_narrow, kMaxBlock, 0, fl.others ? fl.side : stream>>>(e);
+            if (fl.others)
+                k_flat_narrow_other<T, P><<<fl.grid_narrow, kMaxBlock, 0, stream>>>(e);
             launch_gjk(e, stream);
+            cudaEventRecord(fl.join, fl.side);
+            cudaStreamWaitEvent(stream, fl.join, 0);
             const Engine<T, P> &es = s + 1 == e.substeps ? el : e;
             if (e.solve_mode == 1)
                 k_substep<T, P, false><<<fl.grid_solve, 128, fl.substep_smem, stream>>>(es);
@@ -3044,7 +3045,7 @@ namespace rbps_gpu
         cudaError_t rc = run(kKFrame);
         for (int s = 0; s < e.substeps && rc == cudaSuccess; ++s)
         {
-            if (e.gjk_list && (rc = cudaMemsetAsync(e.gjk_count, 0, 4, stream)) != cudaSuccess)
+            if (e.gjk_list && (rc = cudaMemsetAsync(e.gjk_count, 0, 8, stream)) != cudaSuccess)
                 break;
             if ((rc = run(kKNarrow)) != cudaSuccess)
                 break;

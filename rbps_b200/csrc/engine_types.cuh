@@ -253,7 +253,7 @@ namespace rbps_gpu
         // GJK pass (batches with hull colliders): queued (world, candidate)
         // pairs of the current substep and one workspace per k_gjk thread
         uint2 *gjk_list;
-        uint32_t *gjk_count;
+        uint32_t *gjk_count; // queued pairs, then the pass's work counter
         uint32_t gjk_cap, gjk_slots;
         // RBPS_PRECISION_FP32_POS64: per-world origin (3 doubles a world) and
         // the world of every body; body positions are stored relative to it

@@ -9,8 +9,9 @@
 
 namespace rbps_gpu
 {
-    // Warps per CTA of the GJK kernels; each warp owns gjk_warp_bytes of the
-    // CTA's dynamic shared memory.
+    // Warps per CTA of the GJK kernels; each warp owns gjk_warp_bytes (21 KB)
+    // of the CTA's dynamic shared memory.  Eight warps an SM leave a thread
+    // 255 registers, which hold the simplex and both shapes' transforms.
     constexpr int kGjkWarps = 4;
     constexpr size_t kGjkWarpBytes = gjk_warp_bytes<double>();
     constexpr size_t kGjkSmem = kGjkWarps * kGjkWarpBytes;
@@ -25,17 +26,23 @@ namespace rbps_gpu
     // The queued GJK pairs of this substep, one warp per pair, the warp's
     // polytope and clipping buffers in shared memory.
     template <class T, class P>
-    __global__ void __launch_bounds__(kGjkWarps * 32) k_gjk(const Engine<T, P> E)
+    __global__ void __launch_bounds__(kGjkWarps * 32, 2) k_gjk(const Engine<T, P> E)
     {
         extern __shared__ __align__(16) unsigned char gjk_smem[];
         unsigned char *ws = gjk_smem + (threadIdx.x >> 5) * kGjkWarpBytes;
-        const uint32_t warp = blockIdx.x * kGjkWarps + (threadIdx.x >> 5);
+        const uint32_t n = min(E.gjk_count[0], E.gjk_cap);
+        // pairs differ by a hundredfold: after its first (neighbours in the
+        // list on different CTAs) a warp draws each from the pass's counter
+        const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
         const uint32_t n_warps = gridDim.x * kGjkWarps;
-        const uint32_t n = min(*E.gjk_count, E.gjk_cap);
-        for (uint32_t i = warp; i < n; i += n_warps)
+        for (uint32_t i = warp; i < n;)
         {
+            uint32_t next = 0;
+            if (lane_id() == 0)
+                next = atomicAdd(E.gjk_count + 1, 1u); // used after the pair
             const uint2 e = E.gjk_list[i];
             gjk_candidate_warp(E, e.x, e.y, ws);
+            i = n_warps + __shfl_sync(0xffffffffu, next, 0);
         }
     }
 
@@ -123,7 +130,7 @@ namespace rbps_gpu
     }
 
     template <class T, class P>
-    __global__ void __launch_bounds__(kGjkWarps * 32) k_collide(const ShapeDev *sa, const double *ta,
+    __global__ void __launch_bounds__(kGjkWarps * 32, 2) k_collide(const ShapeDev *sa, const double *ta,
                                                                  const ShapeDev *sb, const double *tb,
                                                                  const HullSetDev hulls, uint32_t n, CollideOut *out,
                                                                  int *err)
