@@ -475,7 +475,7 @@ RBPS_API int rbps_bp_configure(rbps_bp *bp, int32_t single_cta, int32_t block_th
  * synchronise the device; hosts that own a fixed device-memory budget).  The
  * SAP sort + sweep of n_objects fat AABBs as a freshly filled broadphase holds
  * them (endpoints in object order), with no allocation: working memory is a
- * file-scope device array of about 2.3 MB per GPU, held until exit.
+ * file-scope device array of about 2.6 MB per GPU, held until exit.
  *   fat_aabbs : device, 6 doubles per object {min.xyz, max.xyz}
  *   user_ids  : device, 1 per object
  *   pairs     : device, 2 * pair_cap; (id_a, id_b), id_a < id_b, in the

@@ -28,11 +28,11 @@ namespace
     template <class Team>
     __global__ void __launch_bounds__(256) k_bp_update(FatBox *fat, uint32_t *ep_key, uint32_t *ep_id,
                                                        uint32_t *ep_pos, uint32_t nbp, uint32_t id_limit,
-                                                       uint32_t pair_cap, int *error, BpScr S)
+                                                       uint32_t pair_cap, int *error, BpScr S, float4 *yz)
     {
         __shared__ BlockShared sh;
         Team tm;
-        const uint32_t n = sap_sort_sweep(tm, fat, ep_key, ep_id, ep_pos, nbp, id_limit, pair_cap, error, S, sh);
+        const uint32_t n = sap_sort_sweep(tm, fat, ep_key, ep_id, ep_pos, nbp, id_limit, pair_cap, error, S, sh, yz);
         if (tm.leader())
             S.misc[kMiscFlags + 5] = n;
     }
@@ -77,6 +77,7 @@ struct rbps_bp
     int *d_err = nullptr;
     std::vector<void *> scratch;
     BpScr S{};
+    float4 *d_yz = nullptr;
     int occ = 0, sms = 0;
     int single_cta = 0;  // run sort + sweep on one CTA (small broadphases)
     int block = 256;
@@ -227,6 +228,11 @@ static int bp_grow(rbps_bp *bp, size_t nobj, size_t npairs)
         bp->scratch.push_back(p);
         *fields[i] = (uint32_t *)p;
     }
+    void *yz;
+    if ((rc = al(&yz, co * sizeof(float4))))
+        return rc;
+    bp->scratch.push_back(yz);
+    bp->d_yz = (float4 *)yz;
     bp->cap_obj = co;
     bp->cap_pairs = cp;
     return RBPS_OK;
@@ -275,7 +281,7 @@ extern "C" int rbps_bp_update(rbps_bp *bp)
         uint32_t cap = (uint32_t)bp->cap_pairs;
         uint32_t id_limit = (uint32_t)(2 * no);
         void *args[] = {&bp->d_fat, &bp->d_key, &bp->d_id, &bp->d_pos, (void *)&nbp, &id_limit, &cap, &bp->d_err,
-                        &bp->S};
+                        &bp->S, &bp->d_yz};
         cudaError_t e = bp->single_cta
                             ? cudaLaunchKernel((const void *)k_bp_update<BlockTeam>, dim3(1), dim3(bp->block), args, 0, 0)
                             : cudaLaunchCooperativeKernel((const void *)k_bp_update<GridTeam>, dim3(grid), dim3(256),

@@ -355,17 +355,15 @@ namespace rbps_gpu
     // pass over the overlap runs that leaves the pairs in the reference's
     // emission order without sorting them.  That order is by the position j
     // of the later opening endpoint, then by the position i of the earlier
-    // one (BroadPhase.cpp:104-152).  The pass counts each j's pairs (hist),
-    // appends every hit (i, j) to a staging list (warp-aggregated slots, so
-    // the list has no particular order) and stores each opening endpoint's
-    // own count in S.cnt.  A scan of hist gives each j its first slot, a
+    // one (BroadPhase.cpp:104-152).  The pass counts each j's pairs (hist)
+    // and appends every hit (i, j) to a staging list (warp-aggregated slots,
+    // so the list has no particular order).  A scan of hist gives each j its first slot, a
     // scatter groups the list by j, and an entry's final slot is its group's
     // first plus the number of the group's entries with a smaller i.  The
     // first min(total, pair_cap) pairs are written to S.pr_a / S.pr_b (pk =
     // j, pv = identity).  Returns the pair count, or ~0u when the hits do not
     // fit the staging lists ((kSmemSortWords - 2 nep) / 2 entries each: 3,104
-    // at the largest nep); S.cnt is complete then, and the caller emits and
-    // sorts in global memory.  Every thread of the CTA must call it.  prof:
+    // at the largest nep); the caller then sweeps in global memory.  Every thread of the CTA must call it.  prof:
     // sub-timers (sweep, pair order), or null.
     template <class SC>
     __device__ __noinline__ uint32_t sweep_staged(const FatBox *fat, const uint32_t *ep_id, const uint32_t *ep_pos,
@@ -390,7 +388,6 @@ namespace rbps_gpu
         for (uint32_t i = t; i < nep; i += B)
         {
             const uint32_t id = ep_id[i];
-            uint32_t c = 0;
             if (!(id & 1u) && id < id_limit)
             {
                 const FatBox fa = fat[id >> 1];
@@ -414,12 +411,10 @@ namespace rbps_gpu
                             if (s < cap)
                                 lst[s] = (i << 16) | j;
                             atomicAdd(&hist[j], 1u);
-                            ++c;
                         }
                     }
                 }
             }
-            S.cnt[i] = c;
         }
         __syncthreads();
         sub_mark(prof, kPhSweep, tclk);
@@ -477,6 +472,181 @@ namespace rbps_gpu
         return total;
     }
 
+    // The sweep in general (grid teams, and CTAs whose endpoints or hits do
+    // not fit the staging area), in one pass.  The opening endpoints are
+    // listed in sweep order (o_pos: their positions; o_end: the first one
+    // that opens after the object has closed; yz: their float y / z extents
+    // rounded outward), so an object's partners are a run of that list.  A
+    // warp takes an object and tests 32 of its run at a time on the 16-byte
+    // extents, read in a row, and the 48-byte double boxes only where those
+    // overlap, so the pairs are exactly those of fat_overlap.  Most tests
+    // fail on y or z: reading boxes by object through the endpoint list,
+    // closing endpoints among them, once to count and once to emit, was most
+    // X  Hits go to S.pr_a / S.pr_b in
+    // no order, a warp's staging block at a time, and are then placed in the
+    // reference's emission order (by the later opening position, then the
+    // earlier one) by counting: a group's first slot plus the number of its
+    // entries with an earlier partner; groups past kGroupMax are radix
+    // sorted instead, which does not grow with their square.
+    constexpr uint32_t kGroupMax = 64;
+    constexpr uint32_t kSweepStage = 128; // hits a warp stages (words of BlockShared::wdig: 8 warps x 256)
+
+    template <class Team, class SC>
+    __device__ __noinline__ uint32_t sweep_runs(const Team &tm, const FatBox *fat, const uint32_t *ep_id,
+                                                const uint32_t *ep_pos, uint32_t nep, uint32_t id_limit,
+                                                uint32_t pair_cap, int *error, const SC &S, BlockShared &sh, float4 *yz)
+    {
+        uint32_t *o_pos = S.ep_k2, *o_end = S.ep_v2; // the sort's second buffers
+        for (uint32_t i = tm.rank(); i < nep; i += tm.size())
+        {
+            const uint32_t id = ep_id[i];
+            S.cnt[i] = !(id & 1u) && id < id_limit ? 1u : 0u;
+        }
+        if (tm.leader())
+        {
+            S.misc[kMiscFlags] = 0u;     // largest group
+            S.misc[kMiscFlags + 4] = 0u; // pairs found
+        }
+        tm.sync();
+        const uint32_t n_open = team_excl_scan(tm, S.cnt, S.cnt, nep, S.tile_sums, sh);
+        for (uint32_t i = tm.rank(); i < nep; i += tm.size())
+        {
+            const uint32_t id = ep_id[i];
+            if ((id & 1u) || id >= id_limit)
+                continue;
+            const uint32_t k = S.cnt[i], end = ep_pos[id + 1];
+            const FatBox f = fat[id >> 1];
+            o_pos[k] = i;
+            o_end[k] = end < nep ? S.cnt[end] : n_open;
+            yz[k] = make_float4(__double2float_rd(f.mn[1]), __double2float_ru(f.mx[1]), __double2float_rd(f.mn[2]),
+                                __double2float_ru(f.mx[2]));
+        }
+        tm.sync();
+        for (uint32_t k = tm.rank(); k <= n_open; k += tm.size())
+            S.cnt[k] = 0u; // cnt[1 + k]: pairs whose later object is k
+        tm.sync();
+        const uint32_t lane = lane_id();
+        uint32_t *stage = sh.wdig + warp_id() * 2 * kSweepStage;
+        uint32_t held = 0;
+        auto flush = [&]() {
+            __syncwarp();
+            uint32_t base = 0;
+            if (lane == 0)
+                base = atomicAdd(&S.misc[kMiscFlags + 4], held);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            for (uint32_t e = lane; e < held; e += 32)
+                if (base + e < pair_cap)
+                {
+                    S.pr_a[base + e] = stage[2 * e];
+                    S.pr_b[base + e] = stage[2 * e + 1];
+                    atomicAdd(&S.cnt[1u + stage[2 * e + 1]], 1u);
+                }
+            held = 0;
+            __syncwarp();
+        };
+        for (uint32_t k = tm.rank() >> 5; k < n_open; k += tm.size() >> 5)
+        {
+            const uint32_t end = o_end[k];
+            if (end <= k + 1)
+                continue;
+            const float4 q = yz[k];
+            const FatBox fa = fat[ep_id[o_pos[k]] >> 1];
+            for (uint32_t j0 = k + 1; j0 < end; j0 += 32)
+            {
+                const uint32_t j = j0 + lane;
+                bool hit = j < end && yz_may_overlap(q, yz[j]);
+                if (hit)
+                    hit = fat_overlap(fa, fat[ep_id[o_pos[j]] >> 1]);
+                const uint32_t m = __ballot_sync(0xffffffffu, hit);
+                if (!m)
+                    continue;
+                if (held + 32u > kSweepStage)
+                    flush();
+                if (hit)
+                {
+                    const uint32_t e = held + __popc(m & ((1u << lane) - 1u));
+                    stage[2 * e] = k;
+                    stage[2 * e + 1] = j;
+                }
+                held += __popc(m);
+            }
+        }
+        if (held)
+            flush();
+        tm.sync();
+        uint32_t total = S.misc[kMiscFlags + 4];
+        if (total > pair_cap)
+        {
+            if (tm.leader())
+                set_error(error, -2);
+            total = pair_cap;
+        }
+        uint32_t group = 0;
+        for (uint32_t k = tm.rank(); k < n_open; k += tm.size())
+            group = max(group, S.cnt[1u + k]);
+        if (group > kGroupMax)
+            atomicMax(&S.misc[kMiscFlags], group);
+        tm.sync();
+        if (S.misc[kMiscFlags] > kGroupMax)
+        {
+            const int bits = n_open > 1 ? 32 - __clz(n_open - 1) : 1;
+            for (uint32_t s = tm.rank(); s < total; s += tm.size())
+            {
+                S.pk[s] = S.pr_a[s];
+                S.pv[s] = s;
+            }
+            tm.sync();
+            team_radix_sort(tm, S.pk, S.pv, S.pk2, S.pv2, total, bits, S.counts, S.tile_sums, sh);
+            for (uint32_t s = tm.rank(); s < total; s += tm.size())
+                S.pk[s] = S.pr_b[S.pv[s]];
+            tm.sync();
+            team_radix_sort(tm, S.pk, S.pv, S.pk2, S.pv2, total, bits, S.counts, S.tile_sums, sh);
+            for (uint32_t s = tm.rank(); s < total; s += tm.size())
+            {
+                S.pr_a[s] = ep_id[o_pos[S.pr_a[s]]] >> 1;
+                S.pr_b[s] = ep_id[o_pos[S.pr_b[s]]] >> 1;
+                S.pk[s] = o_pos[S.pk[s]];
+            }
+        }
+        else
+        {
+            team_excl_scan(tm, S.cnt + 1, S.cnt + 1, n_open, S.tile_sums, sh);
+            // as a group fills, its first slot becomes its end
+            for (uint32_t s = tm.rank(); s < total; s += tm.size())
+            {
+                const uint32_t g = atomicAdd(&S.cnt[1u + S.pr_b[s]], 1u);
+                if (g < total)
+                {
+                    S.pk2[g] = S.pr_a[s];
+                    S.pv2[g] = s;
+                }
+            }
+            tm.sync();
+            for (uint32_t g = tm.rank(); g < total; g += tm.size())
+            {
+                const uint32_t a = S.pk2[g], s = S.pv2[g], b = s < total ? S.pr_b[s] : ~0u;
+                if (a >= n_open || b >= n_open)
+                {
+                    set_error_at(error, kErrInternal, 6, s); // a slot the scatter left unwritten
+                    continue;
+                }
+                const uint32_t g0 = S.cnt[b], g1 = min(total, S.cnt[b + 1u]);
+                uint32_t f = g0;
+                for (uint32_t u = g0; u < g1; ++u)
+                    f += S.pk2[u] < a ? 1u : 0u;
+                if (f < total)
+                {
+                    S.pk[f] = o_pos[b];
+                    S.pv[f] = s;
+                }
+                S.pr_a[s] = ep_id[o_pos[a]] >> 1;
+                S.pr_b[s] = ep_id[o_pos[b]] >> 1;
+            }
+        }
+        tm.sync();
+        return total;
+    }
+
     // Sort + sweep of one SAP state (BroadPhase.cpp:80-152).  On return
     // S.pk / S.pv hold the pairs in the reference emission order (pv indexes
     // the raw object pairs S.pr_a / S.pr_b); returns the pair count.
@@ -484,12 +654,13 @@ namespace rbps_gpu
     // objects leave gaps in the standalone broadphase).  A one-CTA team
     // with the shared staging area sort_smem takes the fast paths above:
     // the merge of the endpoints flagged in `moved` (shared, one word per
-    // endpoint position; null to sort in full) and the single-pass sweep.
+    // endpoint position; null to sort in full) and the staged sweep.  yz:
+    // scratch, one per endpoint pair.
     template <class Team, class SC>
     __device__ __noinline__ uint32_t sap_sort_sweep(const Team &tm, const FatBox *fat, uint32_t *ep_key, uint32_t *ep_id,
                                        uint32_t *ep_pos, uint32_t nbp, uint32_t id_limit, uint32_t pair_cap,
-                                       int *error, const SC &S, BlockShared &sh, uint32_t *sort_smem = nullptr,
-                                       float4 *yz = nullptr, const uint32_t *moved = nullptr,
+                                       int *error, const SC &S, BlockShared &sh, float4 *yz,
+                                       uint32_t *sort_smem = nullptr, const uint32_t *moved = nullptr,
                                        unsigned long long *prof = nullptr)
     {
         const uint32_t nep = 2 * nbp;
@@ -518,20 +689,7 @@ namespace rbps_gpu
                 set_error_at(error, kErrInternal, 4, i); // the endpoint sort must leave the keys ordered
         }
         sub_mark(prof, kPhEndpointSort, tclk);
-        // A grid team's sweep reads every object of an overlap run; most fail
-        // on y or z.  With yz, it first tests 16-byte float extents rounded
-        // outward and reads the 48-byte double box only where they overlap,
-        // so the pairs are exactly those of fat_overlap.
-        const bool pre = tm.ncta() > 1 && yz != nullptr;
-        if (pre)
-            for (uint32_t o = tm.rank(); o < nbp; o += tm.size())
-            {
-                const FatBox f = fat[o];
-                yz[o] = make_float4(__double2float_rd(f.mn[1]), __double2float_ru(f.mx[1]),
-                                    __double2float_rd(f.mn[2]), __double2float_ru(f.mx[2]));
-            }
         tm.sync();
-        bool counted = false;
         if constexpr (kBlock)
             if (staged)
             {
@@ -556,137 +714,12 @@ namespace rbps_gpu
                     tm.sync();
                     return total;
                 }
-                counted = true; // too many pairs to stage: S.cnt holds the counts
             }
-        // count the pairs each opening endpoint emits.  A team spread over
-        // the cooperative grid (one large world) gives each opening endpoint
-        // a warp that tests 32 endpoints of its overlap run at a time: the
-        // runs are long there (hundreds of endpoints) and uneven, so one
-        // thread per endpoint would leave most lanes waiting on a few.
-        const bool by_warp = tm.ncta() > 1;
-        const uint32_t lane = threadIdx.x & 31u;
-        if (by_warp && !counted)
-        {
-            for (uint32_t i = tm.rank() >> 5; i < nep; i += tm.size() >> 5)
-            {
-                const uint32_t id = ep_id[i]; // the same for the whole warp
-                uint32_t c = 0;
-                if (!(id & 1u) && id < id_limit)
-                {
-                    const FatBox fa = fat[id >> 1];
-                    const float4 fq = pre ? yz[id >> 1] : float4{};
-                    const uint32_t end = min(ep_pos[id + 1], nep);
-                    for (uint32_t j0 = i + 1; j0 < end; j0 += 32)
-                    {
-                        const uint32_t j = j0 + lane;
-                        bool hit = false;
-                        if (j < end)
-                        {
-                            const uint32_t id2 = ep_id[j];
-                            hit = !(id2 & 1u) && id2 < id_limit && (!pre || yz_may_overlap(fq, yz[id2 >> 1])) &&
-                                  fat_overlap(fa, fat[id2 >> 1]);
-                        }
-                        c += __popc(__ballot_sync(0xffffffffu, hit));
-                    }
-                }
-                if (lane == 0)
-                    S.cnt[i] = c;
-            }
-        }
-        else if (!counted)
-            for (uint32_t i = tm.rank(); i < nep; i += tm.size())
-            {
-                const uint32_t id = ep_id[i];
-                uint32_t c = 0;
-                if (!(id & 1u) && id < id_limit)
-                {
-                    const FatBox fa = fat[id >> 1];
-                    const uint32_t end = min(ep_pos[id + 1], nep);
-                    for (uint32_t j = i + 1; j < end; ++j)
-                    {
-                        const uint32_t id2 = ep_id[j];
-                        if (!(id2 & 1u) && id2 < id_limit && fat_overlap(fa, fat[id2 >> 1]))
-                            ++c;
-                    }
-                }
-                S.cnt[i] = c;
-            }
-        tm.sync();
-        uint32_t total = team_excl_scan(tm, S.cnt, S.cnt, nep, S.tile_sums, sh);
-        if (tm.leader())
-            S.misc[kMiscFlags + 4] = total; // unclamped pair count
-        if (total > pair_cap)
-        {
-            if (tm.leader())
-                set_error(error, -2);
-            total = pair_cap;
-        }
-        // emit (earlier-opening object, later object, later opening position)
-        if (by_warp)
-        {
-            for (uint32_t i = tm.rank() >> 5; i < nep; i += tm.size() >> 5)
-            {
-                const uint32_t id = ep_id[i];
-                if ((id & 1u) || id >= id_limit)
-                    continue;
-                uint32_t k = S.cnt[i];
-                const FatBox fa = fat[id >> 1];
-                const float4 fq = pre ? yz[id >> 1] : float4{};
-                const uint32_t end = min(ep_pos[id + 1], nep);
-                for (uint32_t j0 = i + 1; j0 < end && k < total; j0 += 32)
-                {
-                    const uint32_t j = j0 + lane;
-                    uint32_t id2 = 0;
-                    bool hit = false;
-                    if (j < end)
-                    {
-                        id2 = ep_id[j];
-                        hit = !(id2 & 1u) && id2 < id_limit && (!pre || yz_may_overlap(fq, yz[id2 >> 1])) &&
-                              fat_overlap(fa, fat[id2 >> 1]);
-                    }
-                    const uint32_t m = __ballot_sync(0xffffffffu, hit);
-                    const uint32_t kk = k + __popc(m & ((1u << lane) - 1u));
-                    if (hit && kk < total)
-                    {
-                        S.pr_a[kk] = id >> 1;
-                        S.pr_b[kk] = id2 >> 1;
-                        S.pk[kk] = j;
-                        S.pv[kk] = kk;
-                    }
-                    k += __popc(m);
-                }
-            }
-        }
-        else
-            for (uint32_t i = tm.rank(); i < nep; i += tm.size())
-            {
-                const uint32_t id = ep_id[i];
-                if ((id & 1u) || id >= id_limit)
-                    continue;
-                uint32_t k = S.cnt[i];
-                const FatBox fa = fat[id >> 1];
-                const uint32_t end = min(ep_pos[id + 1], nep);
-                for (uint32_t j = i + 1; j < end && k < total; ++j)
-                {
-                    const uint32_t id2 = ep_id[j];
-                    if (!(id2 & 1u) && id2 < id_limit && fat_overlap(fa, fat[id2 >> 1]))
-                    {
-                        S.pr_a[k] = id >> 1;
-                        S.pr_b[k] = id2 >> 1;
-                        S.pk[k] = j;
-                        S.pv[k] = k;
-                        ++k;
-                    }
-                }
-            }
-        tm.sync();
+        const uint32_t total = sweep_runs(tm, fat, ep_id, ep_pos, nep, id_limit, pair_cap, error, S, sh, yz);
         sub_mark(prof, kPhSweep, tclk);
-        // reference emission order: stable sort by the later opening position
-        const int bits = nep > 1 ? 32 - __clz(nep - 1) : 1;
-        team_sort_staged(tm, S.pk, S.pv, S.pk2, S.pv2, total, bits, S.counts, S.tile_sums, sh, sort_smem);
         for (uint32_t k = tm.rank(); k + 1 < total; k += tm.size())
             if (S.pk[k] > S.pk[k + 1])
-                set_error_at(error, kErrInternal, 5, k); // pair sort must leave the keys ordered
+                set_error_at(error, kErrInternal, 5, k); // pairs must leave in key order
         tm.sync(); // the caller rewrites S.pk next
         sub_mark(prof, kPhPairOrder, tclk);
         return total;
@@ -756,8 +789,8 @@ namespace rbps_gpu
             }
         }
         tm.sync();
-        return sap_sort_sweep(tm, fat, ep_key, ep_id, ep_pos, nbp, nep, W.pair_cap, E.error, S, sh, sort_smem,
-                              W.n_bodies > kGridWorldBodies ? S.yz : nullptr, moved, prof);
+        return sap_sort_sweep(tm, fat, ep_key, ep_id, ep_pos, nbp, nep, W.pair_cap, E.error, S, sh, S.yz, sort_smem,
+                              moved, prof);
     }
 
     // Filtered SAP pairs followed by the plane candidates; returns the count.

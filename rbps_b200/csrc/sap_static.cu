@@ -57,9 +57,10 @@ namespace
     constexpr uint32_t oPv2 = oPk2 + kPc;
     constexpr uint32_t oMisc = oPv2 + kPc;
     constexpr uint32_t oErr = oMisc + kMiscWords;
-    constexpr uint32_t kScratchWords = oErr + 4;
+    constexpr uint32_t oYz = (oErr + 4 + 3) / 4 * 4; // float4 per object
+    constexpr uint32_t kScratchWords = oYz + 4 * kStaticMaxObjects;
 
-    // The working memory of rbps_sap_pairs_static (about 2.3 MB per GPU).
+    // The working memory of rbps_sap_pairs_static (about 2.6 MB per GPU).
     static __device__ __align__(256) uint32_t g_sap_scratch[kScratchWords];
 
     struct StaticScr
@@ -98,7 +99,8 @@ namespace
         StaticScr S{scratch + oK2, scratch + oV2, scratch + oCounts, scratch + oTileSums, scratch + oCnt,
                     scratch + oPrA, scratch + oPrB, scratch + oPk, scratch + oPv, scratch + oPk2,
                     scratch + oPv2, scratch + oMisc};
-        const uint32_t total = sap_sort_sweep(tm, fat, key, id, pos, n, 2 * n, kStaticMaxPairs, err, S, sh);
+        const uint32_t total = sap_sort_sweep(tm, fat, key, id, pos, n, 2 * n, kStaticMaxPairs, err, S, sh,
+                                              reinterpret_cast<float4 *>(scratch + oYz));
         // sap_sort_sweep ends with a block barrier, so every thread reads the
         // same error word here.  On any error the pairs buffer is left as it
         // was: the pairs kept before an overflow are neither a prefix of the
