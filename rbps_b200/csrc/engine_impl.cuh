@@ -351,20 +351,26 @@ namespace rbps_gpu
         return true;
     }
 
-    // One-CTA fast path of the sweep, in the staging area `smem`: a single
-    // pass over the overlap runs that leaves the pairs in the reference's
-    // emission order without sorting them.  That order is by the position j
-    // of the later opening endpoint, then by the position i of the earlier
-    // one (BroadPhase.cpp:104-152).  The pass counts each j's pairs (hist)
-    // and appends every hit (i, j) to a staging list (warp-aggregated slots,
-    // so the list has no particular order).  A scan of hist gives each j its first slot, a
-    // scatter groups the list by j, and an entry's final slot is its group's
-    // first plus the number of the group's entries with a smaller i.  The
-    // first min(total, pair_cap) pairs are written to S.pr_a / S.pr_b (pk =
-    // j, pv = identity).  Returns the pair count, or ~0u when the hits do not
-    // fit the staging lists ((kSmemSortWords - 2 nep) / 2 entries each: 3,104
-    // at the largest nep); the caller then sweeps in global memory.  Every thread of the CTA must call it.  prof:
-    // sub-timers (sweep, pair order), or null.
+    // One-CTA fast path of the sweep, in the staging area `smem`: sweep_runs
+    // (below) in shared memory.  The opening endpoints are listed in sweep
+    // order with their float y / z extents (rounded outward); a thread takes
+    // an object and walks its run of that list, neighbouring threads on
+    // neighbouring extents; what overlaps goes to a staging list (warp-
+    // aggregated slots, no particular order), and a second pass tests those
+    // few on the double boxes and counts each later object's pairs (hist).  A
+    // scan of hist gives each later object its first slot, a scatter groups
+    // the list, and an entry's final slot is its group's first plus the
+    // number of the group's entries with an earlier partner: the reference's
+    // emission order (BroadPhase.cpp:104-152) without a sort.  The first
+    // min(total, pair_cap) pairs are written to S.pr_a / S.pr_b (pk = the
+    // later position, pv = identity).  Returns the pair count, or ~0u when
+    // the overlaps do not fit the list (3,488 entries at the largest nep);
+    // the caller then sweeps in global memory.  Every thread of the CTA must
+    // call it.  prof: sub-timers (sweep, pair order), or null.
+    // Walking every endpoint of a run, closing ones too, and testing the
+    // 48-byte boxes in the loop was 60-80 % of the frame's broadphase: the
+    // frame of 61 worlds of up to 512 bodies 220 us, 105 us so; of 4,096
+    // worlds 650 and 422 us.
     template <class SC>
     __device__ __noinline__ uint32_t sweep_staged(const FatBox *fat, const uint32_t *ep_id, const uint32_t *ep_pos,
                                                   uint32_t nep, uint32_t id_limit, uint32_t pair_cap, int *error,
@@ -372,15 +378,30 @@ namespace rbps_gpu
                                                   unsigned long long *prof)
     {
         long long tclk = prof ? clock64() : 0;
-        // hist and fill per endpoint, then the two hit lists in what is left
-        const uint32_t cap = (kSmemSortWords - 2 * nep) / 2;
-        uint32_t *hist = smem, *fill = smem + nep;
-        uint32_t *lst = smem + 2 * nep, *grp = lst + cap;
         const uint32_t B = blockDim.x, t = threadIdx.x, lane = t & 31u;
-        for (uint32_t i = t; i < nep; i += B)
+        // each thread a contiguous run of positions
+        const uint32_t per = (nep + B - 1) / B;
+        const uint32_t i0 = min(nep, t * per), i1 = min(nep, i0 + per);
+        auto opens = [&](uint32_t id) { return !(id & 1u) && id < id_limit; };
+        uint32_t mine = 0;
+        for (uint32_t i = i0; i < i1; ++i)
+            mine += opens(ep_id[i]) ? 1u : 0u;
+        uint32_t n_open;
+        uint32_t run = block_excl_scan(mine, sh, &n_open);
+        // position | run end << 16, first slots and fill counts per opening
+        // endpoint; then, in what is left, the extents in the first half and
+        // the list in the second, and the grouped list over the extents
+        // (16-byte aligned) once the sweep is done
+        const uint32_t nb = (n_open + 3u) / 4u * 4u;
+        uint32_t *o_pe = smem, *hist = smem + nb, *fill = smem + 2 * nb, *rest = smem + 3 * nb;
+        const uint32_t cap = (kSmemSortWords - 3 * nb) / 2;
+        float4 *yz = reinterpret_cast<float4 *>(rest);
+        uint32_t *grp = rest, *lst = rest + cap, *rank = lst;
+        static_assert(2 * 4 * (kSmemSortMax / 2) <= kSmemSortWords - 3 * (kSmemSortMax / 2), "the extents' half");
+        for (uint32_t i = i0; i < i1; ++i)
         {
-            hist[i] = 0u;
-            fill[i] = 0u;
+            rank[i] = run;
+            run += opens(ep_id[i]) ? 1u : 0u;
         }
         if (t == 0)
             sh.bcast[3] = 0u;
@@ -388,59 +409,74 @@ namespace rbps_gpu
         for (uint32_t i = t; i < nep; i += B)
         {
             const uint32_t id = ep_id[i];
-            if (!(id & 1u) && id < id_limit)
+            if (!opens(id))
+                continue;
+            const uint32_t k = rank[i], end = ep_pos[id + 1];
+            const FatBox f = fat[id >> 1];
+            o_pe[k] = i | (end < nep ? rank[end] : n_open) << 16;
+            hist[k] = 0u;
+            fill[k] = 0u;
+            yz[k] = make_float4(__double2float_rd(f.mn[1]), __double2float_ru(f.mx[1]), __double2float_rd(f.mn[2]),
+                                __double2float_ru(f.mx[2]));
+        }
+        __syncthreads();
+        for (uint32_t k = t; k < n_open; k += B)
+        {
+            const float4 q = yz[k];
+            const uint32_t end = o_pe[k] >> 16;
+            for (uint32_t j = k + 1; j < end; ++j)
             {
-                const FatBox fa = fat[id >> 1];
-                const uint32_t end = min(ep_pos[id + 1], nep);
-                for (uint32_t j = i + 1; j < end; ++j)
+                const bool hit = yz_may_overlap(q, yz[j]);
+                // one list reservation per warp step, for the lanes that hit
+                const uint32_t act = __activemask();
+                const uint32_t hm = __ballot_sync(act, hit);
+                if (hm)
                 {
-                    const uint32_t id2 = ep_id[j];
-                    const bool hit = !(id2 & 1u) && id2 < id_limit && fat_overlap(fa, fat[id2 >> 1]);
-                    // one list reservation per warp step, for the lanes that hit
-                    const uint32_t act = __activemask();
-                    const uint32_t hm = __ballot_sync(act, hit);
-                    if (hm)
-                    {
-                        const uint32_t leader = __ffs(hm) - 1;
-                        uint32_t s = 0;
-                        if (lane == leader)
-                            s = atomicAdd(&sh.bcast[3], (uint32_t)__popc(hm));
-                        s = __shfl_sync(act, s, leader) + __popc(hm & ((1u << lane) - 1u));
-                        if (hit)
-                        {
-                            if (s < cap)
-                                lst[s] = (i << 16) | j;
-                            atomicAdd(&hist[j], 1u);
-                        }
-                    }
+                    const uint32_t leader = __ffs(hm) - 1;
+                    uint32_t s = 0;
+                    if (lane == leader)
+                        s = atomicAdd(&sh.bcast[3], (uint32_t)__popc(hm));
+                    s = __shfl_sync(act, s, leader) + __popc(hm & ((1u << lane) - 1u));
+                    if (hit && s < cap)
+                        lst[s] = k << 16 | j;
                 }
             }
         }
         __syncthreads();
-        sub_mark(prof, kPhSweep, tclk);
-        const uint32_t total = sh.bcast[3];
-        if (total > cap)
+        const uint32_t listed = sh.bcast[3];
+        if (listed > cap)
             return ~0u;
-        // first slot of each j
-        const uint32_t per = (nep + B - 1) / B;
-        const uint32_t i0 = min(nep, t * per), i1 = min(nep, i0 + per);
-        uint32_t mine = 0;
-        for (uint32_t i = i0; i < i1; ++i)
-            mine += hist[i];
-        uint32_t sum;
-        uint32_t run = block_excl_scan(mine, sh, &sum);
-        for (uint32_t i = i0; i < i1; ++i)
+        auto object = [&](uint32_t k) { return ep_id[o_pe[k] & 0xffffu] >> 1; };
+        for (uint32_t s = t; s < listed; s += B)
         {
-            const uint32_t h = hist[i];
-            hist[i] = run;
+            const uint32_t v = lst[s];
+            if (fat_overlap(fat[object(v >> 16)], fat[object(v & 0xffffu)]))
+                atomicAdd(&hist[v & 0xffffu], 1u);
+            else
+                lst[s] = ~0u;
+        }
+        __syncthreads();
+        sub_mark(prof, kPhSweep, tclk);
+        // first slot of each later object
+        const uint32_t pk = (n_open + B - 1) / B;
+        const uint32_t k0 = min(n_open, t * pk), k1 = min(n_open, k0 + pk);
+        mine = 0;
+        for (uint32_t k = k0; k < k1; ++k)
+            mine += hist[k];
+        uint32_t total;
+        run = block_excl_scan(mine, sh, &total);
+        for (uint32_t k = k0; k < k1; ++k)
+        {
+            const uint32_t h = hist[k];
+            hist[k] = run;
             run += h;
         }
-        if (t == 0 && sum != total)
-            set_error_at(error, kErrInternal, 6, total); // the two counts of one pass must agree
         __syncthreads();
-        for (uint32_t s = t; s < total; s += B)
+        for (uint32_t s = t; s < listed; s += B)
         {
             const uint32_t v = lst[s], j = v & 0xffffu;
+            if (v == ~0u)
+                continue;
             const uint32_t g = hist[j] + atomicAdd(&fill[j], 1u);
             if (g < total)
                 grp[g] = v;
@@ -449,8 +485,8 @@ namespace rbps_gpu
         const uint32_t n_out = min(total, pair_cap);
         for (uint32_t s = t; s < total; s += B)
         {
-            const uint32_t v = grp[s], i = v >> 16, j = v & 0xffffu;
-            if (i >= nep || j >= nep)
+            const uint32_t v = grp[s], k = v >> 16, j = v & 0xffffu;
+            if (k >= n_open || j >= n_open)
             {
                 set_error_at(error, kErrInternal, 6, v); // a slot the scatter left unwritten
                 continue;
@@ -458,12 +494,12 @@ namespace rbps_gpu
             const uint32_t g0 = hist[j], g1 = min(total, g0 + fill[j]);
             uint32_t f = g0;
             for (uint32_t u = g0; u < g1; ++u)
-                f += (grp[u] >> 16) < i ? 1u : 0u;
+                f += (grp[u] >> 16) < k ? 1u : 0u;
             if (f < n_out)
             {
-                S.pr_a[f] = ep_id[i] >> 1;
-                S.pr_b[f] = ep_id[j] >> 1;
-                S.pk[f] = j;
+                S.pr_a[f] = object(k);
+                S.pr_b[f] = object(j);
+                S.pk[f] = o_pe[j] & 0xffffu;
                 S.pv[f] = f;
             }
         }
@@ -1941,7 +1977,7 @@ namespace rbps_gpu
     __global__ void __launch_bounds__(kMaxBlock, RBPS_FRAME_MIN_BLOCKS) k_phase_frame(const Engine<T, P> E, uint32_t ctr)
     {
         __shared__ BlockShared sh;
-        __shared__ uint32_t sort_smem[kSmemSortWords];
+        __shared__ __align__(16) uint32_t sort_smem[kSmemSortWords];
         BlockTeam tm;
         each_small_world(E.small_worlds, E.n_small, E.work_counter + ctr,
                          [&](uint32_t w) { phase_frame(E, tm, w, sh, sort_smem); });
