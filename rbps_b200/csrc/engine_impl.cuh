@@ -1438,18 +1438,40 @@ namespace rbps_gpu
         store_vel(B, bb, Bb);
     }
 
+    // The same with a pair of lanes, a body each (solver.cuh).
     template <class T, class P>
-    __device__ __forceinline__ void solve_cand_position(const Engine<T, P> &E, const WorldDev &W, const Cand &cd,
-                                                        CandContacts<T, P> &cc)
+    __device__ __forceinline__ void solve_pair_position_split(const Bodies<T, P> &B, uint32_t ba, uint32_t bb,
+                                                              CandContacts<T, P> &cc)
     {
-        solve_pair_position(E.B, E.inv_h, W.body_off + cd.ba, W.body_off + cd.bb, cc);
+        const int n = cc.n;
+        if (n == 0)
+            return;
+        const PairLane pl;
+        const vec3<T> nrm = v3(cc.normal);
+        const T sf = cc.mat.y;
+        const uint32_t i = pl.b ? bb : ba;
+        BodyR<T, P> X;
+        load_body(B, i, X, true);
+        for (int k = 0; k < n; ++k)
+            contact_position_split(X, pl, nrm, sf, cc.pt[k]);
+        store_pose(B, i, X);
     }
 
     template <class T, class P>
-    __device__ __forceinline__ void solve_cand_velocity(const Engine<T, P> &E, const WorldDev &W, const Cand &cd,
-                                                        const CandContacts<T, P> &cc)
+    __device__ __forceinline__ void solve_pair_velocity_split(const Bodies<T, P> &B, T h, uint32_t ba, uint32_t bb,
+                                                              const CandContacts<T, P> &cc)
     {
-        solve_pair_velocity(E.B, E.h, W.body_off + cd.ba, W.body_off + cd.bb, cc);
+        const int n = cc.n;
+        if (n == 0)
+            return;
+        const PairLane pl;
+        const vec3<T> nrm = v3(cc.normal);
+        const uint32_t i = pl.b ? bb : ba;
+        BodyR<T, P> X;
+        load_body(B, i, X, false);
+        for (int k = 0; k < n; ++k)
+            contact_velocity_split(X, pl, nrm, cc.mat.x, cc.mat.z, cc.pt[k], h);
+        store_vel(B, i, X);
     }
 
     template <class T, class P>
@@ -1642,7 +1664,8 @@ namespace rbps_gpu
     // Tangled worlds end in dozens of such colours (a body with 60 contacts
     // needs 60 colours, most of them nearly empty), and a grid barrier costs
     // several block barriers.
-    template <class Team, class F>
+    // Lanes: consecutive threads that take a slot together.
+    template <int Lanes = 1, class Team, class F>
     __device__ __forceinline__ void sweep_colors(const Team &tm, const uint32_t *off, uint32_t n, F &&solve)
     {
         constexpr bool kGrid = std::is_same<Team, GridTeam>::value;
@@ -1652,7 +1675,7 @@ namespace rbps_gpu
             // skip test for empty colours measured 0.4 % slower here)
             for (uint32_t col = 0; col < n; ++col)
             {
-                for (uint32_t q = off[col] + tm.rank(); q < off[col + 1]; q += tm.size())
+                for (uint32_t q = off[col] + tm.rank() / Lanes; q < off[col + 1]; q += tm.size() / Lanes)
                     solve(q);
                 tm.sync();
             }
@@ -1660,7 +1683,7 @@ namespace rbps_gpu
         }
         uint32_t tail = n;
         if constexpr (kGrid)
-            while (tail > 0 && off[tail] - off[tail - 1] <= blockDim.x)
+            while (tail > 0 && off[tail] - off[tail - 1] <= blockDim.x / Lanes)
                 --tail;
         for (uint32_t col = 0; col < n; ++col)
         {
@@ -1670,7 +1693,7 @@ namespace rbps_gpu
             if (!on_cta || blockIdx.x == 0)
             {
                 const uint32_t r = on_cta ? threadIdx.x : tm.rank(), step = on_cta ? blockDim.x : tm.size();
-                for (uint32_t q = off[col] + r; q < off[col + 1]; q += step)
+                for (uint32_t q = off[col] + r / Lanes; q < off[col + 1]; q += step / Lanes)
                     solve(q);
             }
             if (on_cta)
@@ -1680,6 +1703,56 @@ namespace rbps_gpu
         }
         if (kGrid && tail < n)
             tm.sync();
+    }
+
+    // The contacts of both solves with a pair of lanes a candidate
+    // (kSplitPairs), in the same order as the one-lane loops below: relax(c,
+    // ba, bb) for candidate c of world-local bodies ba and bb.
+    template <bool Ref, class T, class P, class Team, class F>
+    __device__ __forceinline__ void relax_split(const Team &tm, const Scr<T, P> &S, const uint32_t *book,
+                                                const uint2 *slots, F &&relax)
+    {
+        auto in_order = [&](uint32_t q) {
+            const uint32_t c = S.corder[q];
+            const Cand cd = S.cand[c];
+            relax(c, cd.ba, cd.bb);
+        };
+        if constexpr (Ref)
+        {
+            uint32_t n_lvl;
+            const uint32_t *loff = level_offsets(S, book, n_lvl);
+            sweep_colors<2>(tm, loff, n_lvl, in_order);
+        }
+        else
+        {
+            const uint32_t *coff = book ? book + 66 : S.misc + kMiscCOff;
+            const uint32_t n_colors = book ? book[132] : S.misc[kMiscNColors];
+            const bool sl = slots && book && book[133];
+            sweep_colors<2>(tm, coff, n_colors, [&](uint32_t q) {
+                uint32_t c, ba, bb;
+                slot_entry(S, book, sl ? slots : nullptr, q, c, ba, bb);
+                relax(c, ba, bb);
+            });
+            if (coff[kColorSerial + 1] > coff[kColorSerial])
+            {
+                uint32_t serial0 = coff[kColorSerial];
+                if (!book)
+                {
+                    const uint32_t *c2 = S.misc + kMiscC2Off;
+                    sweep_colors<2>(tm, c2, kColorSerial, in_order);
+                    serial0 = c2[kColorSerial];
+                }
+                if (tm.rank() < 2)
+                    for (uint32_t q = serial0; q < coff[kColorSerial + 1]; ++q)
+                    {
+                        const uint32_t c = sl ? slots[q].x : S.corder[q];
+                        const Cand cd = S.cand[c];
+                        relax(c, cd.ba, cd.bb);
+                        __syncwarp(3u << (threadIdx.x & 30u)); // the next may read the other lane's body
+                    }
+                tm.sync();
+            }
+        }
     }
 
     // Ref: the reference's order, level by level (schedule_levels), else
@@ -1692,7 +1765,10 @@ namespace rbps_gpu
         const Scr<T, P> S = world_scratch(E, W);
         PhaseClock clk(prof_slots(E, tm, w), false);
         const uint32_t shift = W.body_off - boff; // joint body ids are batch-global
-        if constexpr (Ref)
+        if constexpr (kSplitPairs<T>)
+            relax_split<Ref>(tm, S, book, slots,
+                             [&](uint32_t c, uint32_t ba, uint32_t bb) { solve_pair_position_split(B, boff + ba, boff + bb, S.cc[c]); });
+        else if constexpr (Ref)
         {
             uint32_t n_lvl;
             const uint32_t *loff = level_offsets(S, book, n_lvl);
@@ -1764,12 +1840,16 @@ namespace rbps_gpu
             const uint32_t *jco = E.jcolor_off + W.jc_off;
             for (uint32_t jc = 0; jc < W.n_jcolors; ++jc)
             {
-                for (uint32_t q = jco[jc] + tm.rank(); q < jco[jc + 1]; q += tm.size())
+                constexpr uint32_t kLanes = kSplitPairs<T> ? 2 : 1;
+                for (uint32_t q = jco[jc] + tm.rank() / kLanes; q < jco[jc + 1]; q += tm.size() / kLanes)
                 {
                     Joint<T> jt = E.joints[W.joint_off + E.jorder[q]];
                     jt.b1 -= shift;
                     jt.b2 -= shift;
-                    solve_joint_rows(B, jt, joint_rows(E, jt), E.inv_h);
+                    if constexpr (kSplitPairs<T>)
+                        solve_joint_rows_split(B, jt, joint_rows(E, jt), E.inv_h);
+                    else
+                        solve_joint_rows(B, jt, joint_rows(E, jt), E.inv_h);
                 }
                 tm.sync();
             }
@@ -1799,7 +1879,10 @@ namespace rbps_gpu
         const Scr<T, P> S = world_scratch(E, W);
         PhaseClock clk(prof_slots(E, tm, w), false);
         const uint32_t shift = W.body_off - boff;
-        if constexpr (Ref)
+        if constexpr (kSplitPairs<T>)
+            relax_split<Ref>(tm, S, book, slots,
+                             [&](uint32_t c, uint32_t ba, uint32_t bb) { solve_pair_velocity_split(B, E.h, boff + ba, boff + bb, S.cc[c]); });
+        else if constexpr (Ref)
         {
             uint32_t n_lvl;
             const uint32_t *loff = level_offsets(S, book, n_lvl);

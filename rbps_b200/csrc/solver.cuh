@@ -710,6 +710,246 @@ namespace rbps_gpu
         store_pose(B, j.b2, b2);
     }
 
+    // ------------------------------------------------------- a lane per body
+    // The rows above with a pair of lanes a row, the even lane body 1 (A) and
+    // the odd lane body 2 (B): each holds its own body, and the lanes swap
+    // what a row needs of both (points, velocities, inverse masses).  A row
+    // is a long chain with little to overlap, and one lane issues both
+    // bodies' arithmetic one instruction after another: in double, 3.3
+    // cycles each, the issue was longer than the chain.  The values are those
+    // of the one-lane rows, each computed by the same operations; in double,
+    // without FMA contraction, the bits are too, so only double takes these
+    // (float contracts differently in another function).  96 worlds of
+    // jointed chains in reference order: 12 joint levels 86 us a substep with
+    // a lane a joint and 54 us with two, contacts of the larger 71 and 47 us.
+    template <class T> constexpr bool kSplitPairs = sizeof(T) == 8;
+
+    struct PairLane
+    {
+        bool b;        // this lane holds body 2 (B)
+        unsigned mask; // the pair's two lanes
+        __device__ __forceinline__ PairLane() : b(threadIdx.x & 1u), mask(3u << (threadIdx.x & 30u)) {}
+        template <class T> __device__ __forceinline__ T other(T v) const { return __shfl_xor_sync(mask, v, 1); }
+        template <class T> __device__ __forceinline__ vec3<T> other(const vec3<T> &v) const
+        {
+            return {other(v.x), other(v.y), other(v.z)};
+        }
+        // A's value less B's, the same on both lanes
+        template <class T> __device__ __forceinline__ vec3<T> a_minus_b(const vec3<T> &own) const
+        {
+            const vec3<T> o = other(own);
+            return b ? o - own : own - o;
+        }
+        // before a lane writes what the other has read
+        __device__ __forceinline__ void sync() const { __syncwarp(mask); }
+    };
+
+    // contact_position
+    template <class T, class P>
+    __device__ __forceinline__ void contact_position_split(BodyR<T, P> &X, const PairLane &pl, const vec3<T> &n,
+                                                           T static_friction, ContactPt<T, P> &c)
+    {
+        const vec3<T> rl = v3(pl.b ? c.rb : c.ra);
+        V4<P> &cp = pl.b ? c.pb : c.pa;
+        T lam_n = c.lam_n, lam_t = c.lam_t, vrel;
+        const vec3<T> p = X.x + rotate(X.q, rl);
+        const T d = dot(pl.a_minus_b(p), n);
+        if (d <= T(0.0))
+        {
+            cp = V4<P>{P(p.x), P(p.y), P(p.z), P(0)};
+            if (!pl.b)
+                c.coll = 0;
+            return;
+        }
+        const vec3<T> r = p - X.x;
+        vrel = dot(pl.a_minus_b(X.v + cross(X.w, r)), n);
+        {
+            smat3<T> I;
+            const T w = pos_w(X, r, n, I);
+            const T denom = w + pl.other(w);
+            if (!(denom < T(kEpsilon)))
+            {
+                const T dl = div_guarded(-d, denom);
+                lam_n += dl;
+                if (lam_n > T(0.0))
+                    lam_n = T(0.0);
+                const vec3<T> imp = dl * n;
+                pos_impulse(X, I, pl.b ? -imp : imp, r);
+            }
+        }
+        const vec3<T> r_wc = rotate(X.q, rl);
+        const vec3<T> cur = X.x + r_wc;
+        cp = V4<P>{P(cur.x), P(cur.y), P(cur.z), P(0)};
+        const vec3<T> prev = X.xp + rotate(X.qp, rl);
+        const vec3<T> dp = pl.a_minus_b(cur - prev);
+        const vec3<T> dpt = dp - dot(dp, n) * n;
+        const T slip = length(dpt);
+        if (!(slip < T(kEpsilon)))
+        {
+            const vec3<T> t = normalize(dpt);
+            smat3<T> I;
+            const T w = pos_w(X, r_wc, t, I);
+            const T denom = w + pl.other(w);
+            if (!(denom < T(kEpsilon)))
+            {
+                const T dl = div_guarded(-slip, denom);
+                const T old = lam_t;
+                lam_t += dl;
+                const T cone = static_friction * lam_n;
+                if (lam_t < cone)
+                    lam_t = cone;
+                const T actual = lam_t - old;
+                if (!(rabs(actual) < T(kEpsilon)))
+                {
+                    const vec3<T> imp = actual * t;
+                    pos_impulse(X, I, pl.b ? -imp : imp, r_wc);
+                }
+            }
+        }
+        pl.sync();
+        if (!pl.b)
+        {
+            c.coll = 1;
+            c.vrel = vrel;
+            c.lam_n = lam_n;
+            c.lam_t = lam_t;
+        }
+    }
+
+    // contact_velocity
+    template <class T, class P>
+    __device__ __forceinline__ void contact_velocity_split(BodyR<T, P> &X, const PairLane &pl, const vec3<T> &n,
+                                                           T restitution, T dynamic_friction,
+                                                           const ContactPt<T, P> &c, T h)
+    {
+        if (!c.coll)
+            return;
+        const vec3<T> r = vec3<T>(v3(pl.b ? c.pb : c.pa)) - X.x;
+        const vec3<T> v_rel = pl.a_minus_b(X.v + cross(X.w, r));
+        const T v_n = dot(v_rel, n);
+        const vec3<T> v_t = v_rel - n * v_n;
+        const T v_t_mag = length(v_t);
+        T e = restitution;
+        if (rabs(c.vrel) <= T(2.0 * 9.8) * h)
+            e = T(0.0);
+        const T v_n_target = rmin(-e * c.vrel, T(0.0));
+        const T dv_n = v_n_target - v_n;
+        T dv_t = T(0.0);
+        if (v_t_mag > T(kEpsilon))
+        {
+            const T limit = div_guarded(dynamic_friction * rabs(c.lam_n), h);
+            dv_t = -rmin(limit, v_t_mag);
+        }
+        smat3<T> I;
+        const T w_n = pos_w(X, r, n, I);
+        const T denom_n = w_n + pl.other(w_n);
+        if (denom_n > T(kEpsilon) && rabs(dv_n) > T(kEpsilon))
+        {
+            const vec3<T> imp = div_guarded(dv_n, denom_n) * n;
+            pos_vel_impulse(X, I, pl.b ? -imp : imp, r);
+        }
+        if (v_t_mag > T(kEpsilon) && rabs(dv_t) > T(kEpsilon))
+        {
+            const vec3<T> t = v_t * div_guarded(T(1.0), v_t_mag);
+            const T w_t = pos_w(X, r, t, I);
+            const T denom_t = w_t + pl.other(w_t);
+            if (denom_t > T(kEpsilon))
+            {
+                const vec3<T> imp = div_guarded(dv_t, denom_t) * t;
+                pos_vel_impulse(X, I, pl.b ? -imp : imp, r);
+            }
+        }
+    }
+
+    // solve_row; r is the lane's own copy of the row, updated on both
+    template <class T, class P>
+    __device__ __forceinline__ void solve_row_split(BodyR<T, P> &X, const PairLane &pl, Row<T> &r, T inv_h)
+    {
+        const vec3<T> dir = v3(r.dir);
+        smat3<T> I;
+        if (r.type == kRowRotational)
+        {
+            const T w = rot_w(X, dir, I), wo = pl.other(w);
+            const T dl = row_delta_lambda(r, pl.b ? wo : w, pl.b ? w : wo, inv_h);
+            r.r2.w += dl;
+            const vec3<T> imp = dl * dir;
+            rot_impulse(X, I, pl.b ? -imp : imp);
+        }
+        else
+        {
+            const vec3<T> rr = rotate(X.q, v3(pl.b ? r.r2 : r.r1));
+            const T w = pos_w(X, rr, dir, I), wo = pl.other(w);
+            const T dl = row_delta_lambda(r, pl.b ? wo : w, pl.b ? w : wo, inv_h);
+            r.r2.w += dl;
+            const vec3<T> imp = dl * dir;
+            pos_impulse(X, I, pl.b ? -imp : imp, rr);
+        }
+    }
+
+    // solve_ball_joint
+    template <class T, class P>
+    __device__ __forceinline__ void solve_ball_joint_split(BodyR<T, P> &X, const PairLane &pl, const Joint<T> &j,
+                                                           Row<T> *rows, T inv_h)
+    {
+        Row<T> r0 = rows[0], r1 = rows[1];
+        r0.r2.w = T(0.0);
+        row_set_value_div(r0, pl.a_minus_b(X.x + rotate(X.q, v3(pl.b ? j.r2 : j.r1))));
+        solve_row_split(X, pl, r0, inv_h);
+        vec3<T> err_limit(T(0.0), T(0.0), T(0.0));
+        if (j.limited)
+        {
+            const vec3<T> own = rotate(X.q, v3(j.axis)), oth = pl.other(own);
+            const vec3<T> a1 = pl.b ? oth : own, a2 = pl.b ? own : oth;
+            const vec3<T> c = cross(a1, a2);
+            const T phi = atan2(length(c), dot(a1, a2));
+            if (phi < j.lower || phi > j.upper)
+            {
+                const bool lo = phi < j.lower;
+                const T s = lo ? j.sin_lo : j.sin_hi;
+                const T co = lo ? j.cos_lo : j.cos_hi;
+                const vec3<T> nn = normalize(normalize(c));
+                const quat<T> rq(co, nn.x * s, nn.y * s, nn.z * s);
+                err_limit = cross(rotate(rq, a1), a2);
+            }
+        }
+        r1.r2.w = T(0.0);
+        row_set_value_div(r1, -err_limit);
+        solve_row_split(X, pl, r1, inv_h);
+        pl.sync();
+        if (!pl.b)
+        {
+            rows[0] = r0;
+            rows[1] = r1;
+        }
+    }
+
+    // solve_joint_rows
+    template <class T, class P>
+    __device__ __noinline__ void solve_joint_rows_split(const Bodies<T, P> &B, const Joint<T> &j, Row<T> *rows, T inv_h)
+    {
+        const PairLane pl;
+        const uint32_t i = pl.b ? j.b2 : j.b1;
+        BodyR<T, P> X;
+        load_body(B, i, X, false);
+        if (j.type == kSpherical)
+            solve_ball_joint_split(X, pl, j, rows, inv_h);
+        else
+        {
+            Row<T> next = rows[0];
+            for (int r = 0; r < j.count; ++r)
+            {
+                Row<T> cur = next;
+                if (r + 1 < j.count)
+                    next = rows[r + 1]; // on its way while this one is solved
+                solve_row_split(X, pl, cur, inv_h);
+                pl.sync();
+                if (!pl.b)
+                    rows[r].r2.w = cur.r2.w;
+            }
+        }
+        store_pose(B, i, X);
+    }
+
     // apply_{prismatic,revolute}_joint_damping (Joint.cpp:184-220)
     template <class T, class P>
     __device__ __noinline__ void joint_damping(const Bodies<T, P> &B, const Joint<T> &j, T h)
