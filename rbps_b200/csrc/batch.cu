@@ -1533,6 +1533,7 @@ static int commit_typed(rbps_batch *b)
         CU(occupancy_flat<T, P>(2, kMaxBlockHost, &per_sm, 0));
         b->flat.grid_sort = std::max(1, per_sm) * b->sm_count;
         b->flat.block_solve = 128;
+        b->flat.sm_count = b->sm_count;
         if ((rc = set_team_split<T, P>(b, kBlockTeamBodies, kPairTeamBodies)))
             return rc;
         // side stream + events for the parallel narrowphase kernels

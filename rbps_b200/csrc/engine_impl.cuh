@@ -1426,6 +1426,20 @@ namespace rbps_gpu
                                                         const CandContacts<T, P> &cc)
     {
         const int n = cc.n;
+        // what a row reads of its point, a point ahead: the block comes from
+        // L2, and a load behind the count or the last row waits for it alone
+        // (61 worlds, two steps: 2.15 ms without, 2.10 so; the position rows,
+        // which hold more registers, gained nothing by it)
+        ContactPt<T, P> next;
+        auto fetch = [&](int k) {
+            const ContactPt<T, P> &c = cc.pt[k];
+            next.pa = c.pa;
+            next.pb = c.pb;
+            next.lam_n = c.lam_n;
+            next.vrel = c.vrel;
+            next.coll = c.coll;
+        };
+        fetch(0);
         if (n == 0)
             return;
         const vec3<T> nrm = v3(cc.normal);
@@ -1433,7 +1447,12 @@ namespace rbps_gpu
         load_body(B, ba, A, false);
         load_body(B, bb, Bb, false);
         for (int k = 0; k < n; ++k)
-            contact_velocity(A, Bb, nrm, cc.mat.x, cc.mat.z, cc.pt[k], h);
+        {
+            const ContactPt<T, P> c = next;
+            if (k + 1 < n)
+                fetch(k + 1);
+            contact_velocity(A, Bb, nrm, cc.mat.x, cc.mat.z, c, h);
+        }
         store_vel(B, ba, A);
         store_vel(B, bb, Bb);
     }
@@ -2808,10 +2827,14 @@ namespace rbps_gpu
 #ifndef RBPS_SUBSTEP_MIN_BLOCKS
 #define RBPS_SUBSTEP_MIN_BLOCKS 4
 #endif
-// In double a pair's two bodies alone take 104 registers: two CTAs (255).
-#ifndef RBPS_SUBSTEP_MIN_BLOCKS_F64
-#define RBPS_SUBSTEP_MIN_BLOCKS_F64 2
-#endif
+    // In double a pair's two bodies alone take 104 registers: two CTAs (255).
+    template <class T> constexpr int kSubstepBlocks = sizeof(T) == 8 ? 2 : RBPS_SUBSTEP_MIN_BLOCKS;
+    // A launch whose CTAs are all resident at three an SM gains nothing from
+    // a fourth slot, and at 168 registers a float row spills nothing: 61
+    // worlds of up to 512 bodies, two steps, 2.10 ms at 128 registers and
+    // 1.99 at 168; 256 towers of 64 boxes 2.51 and 2.26 (two CTAs, 255
+    // registers: 1.99 and 2.25).
+    constexpr int kSubstepBlocksFew = 3;
     // The rest of a substep for every small world: colouring, integrate
     // (Body.cpp:18-39), position solve + velocity update, velocity solve.
     // The largest worlds (the first n_block_worlds of the list) get a whole
@@ -3003,9 +3026,8 @@ namespace rbps_gpu
     // barrier is the team's own.  Dynamic shared memory: E.smem_cap_block
     // bodies for a CTA world, E.smem_cap_pair for each of two half-CTA
     // worlds, or E.smem_cap_warp for each of four warp worlds.
-    template <class T, class P, bool Ref>
-    __global__ void __launch_bounds__(128, sizeof(T) == 8 ? RBPS_SUBSTEP_MIN_BLOCKS_F64 : RBPS_SUBSTEP_MIN_BLOCKS)
-        k_substep(const Engine<T, P> E)
+    template <class T, class P, bool Ref, int MinBlocks>
+    __global__ void __launch_bounds__(128, MinBlocks) k_substep(const Engine<T, P> E)
     {
         __shared__ ScanShared sh; // the colouring's compaction scans are all the teams need
         extern __shared__ __align__(16) unsigned char smem[];
@@ -3097,10 +3119,14 @@ namespace rbps_gpu
                 rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
             return rc;
         };
-        cudaError_t rc = open(k_substep<T, P, false>);
+        cudaError_t rc = open(k_substep<T, P, false, kSubstepBlocks<T>>);
         if constexpr (sizeof(T) == 8)
+        {
             if (rc == cudaSuccess)
-                rc = open(k_substep<T, P, true>);
+                rc = open(k_substep<T, P, true, kSubstepBlocks<T>>);
+        }
+        else if (rc == cudaSuccess)
+            rc = open(k_substep<T, P, false, kSubstepBlocksFew>);
         return rc;
     }
 
@@ -3144,9 +3170,15 @@ namespace rbps_gpu
             cudaStreamWaitEvent(stream, fl.join, 0);
             const Engine<T, P> &es = s + 1 == e.substeps ? el : e;
             if (e.solve_mode == 1)
-                k_substep<T, P, false><<<fl.grid_solve, 128, fl.substep_smem, stream>>>(es);
+            {
+                auto *kernel = k_substep<T, P, false, kSubstepBlocks<T>>;
+                if constexpr (sizeof(T) == 4)
+                    if (fl.grid_solve <= kSubstepBlocksFew * fl.sm_count)
+                        kernel = k_substep<T, P, false, kSubstepBlocksFew>;
+                kernel<<<fl.grid_solve, 128, fl.substep_smem, stream>>>(es);
+            }
             else if constexpr (sizeof(T) == 8)
-                k_substep<T, P, true><<<fl.grid_solve, 128, fl.substep_smem, stream>>>(es);
+                k_substep<T, P, true, kSubstepBlocks<T>><<<fl.grid_solve, 128, fl.substep_smem, stream>>>(es);
             else
             {
                 k_ref_levels<T, P><<<e.n_small, 128, 0, stream>>>(es);
@@ -3174,7 +3206,7 @@ namespace rbps_gpu
             *blocks_per_sm = a < b ? a : b;
             return rc;
         }
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_substep<T, P, false>, block, fl_smem);
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_substep<T, P, false, kSubstepBlocks<T>>, block, fl_smem);
     }
 
     // Enqueues one step of one large world: 2 + 4 * substeps cooperative

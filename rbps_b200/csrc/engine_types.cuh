@@ -303,6 +303,7 @@ namespace rbps_gpu
     struct FlatLaunch
     {
         int grid_narrow, grid_solve, block_solve;
+        int sm_count;
         int grid_sort;       // the class-sort kernels: every CTA they can keep resident
         size_t substep_smem; // dynamic shared memory of k_substep
         bool triangles, others; // the batch has meshes or heightmaps / other kinds beyond sphere, box, capsule, plane
