@@ -2324,6 +2324,24 @@ namespace rbps_gpu
         }
     }
 
+    // The warp's turn in a range dealt out in chunks: consecutive chunks go to
+    // different CTAs, so a range of few chunks still meets every SM (with the
+    // CTA's warps in a row, 536 chunks of 32 sat on 67 of 148).
+    __device__ __forceinline__ uint32_t narrow_warp() { return (threadIdx.x >> 5) * gridDim.x + blockIdx.x; }
+
+    // Double batches are few and small: a range that does not fill half the
+    // grid's warps 32 deep is dealt evenly over them, down to one entry a
+    // warp, as a warp's time is the sum of its lanes' branches (the box-box
+    // axes and clipping above all).  512 bodies, box-box: 26.8 us a launch at
+    // 32 a warp and 80 registers, 15.4 so.  In float, with thousands of pairs
+    // and three CTAs an SM, dealing evenly only spreads each thread's
+    // 848-byte stack over more L1 (256 towers: 27 and 43 us).
+    __device__ __forceinline__ uint32_t narrow_share(uint32_t per_warp, uint32_t n, uint32_t n_warps)
+    {
+        const uint32_t half = n_warps / 2, even = (n + half - 1) / half;
+        return even < 32u ? max(even, 1u) : per_warp;
+    }
+
     // Narrowphase of every candidate of the small worlds but the box-box
     // ones, in class order.
     // Entries [0, n) of a class-sorted range are dealt to the grid's warps
@@ -2339,16 +2357,20 @@ namespace rbps_gpu
 #ifndef RBPS_NARROW_MIN_BLOCKS
 #define RBPS_NARROW_MIN_BLOCKS 3
 #endif
+    // In double 80 registers spill up to 7 KB a thread: one CTA (255).
+    template <class T> constexpr int kNarrowBlocks = sizeof(T) == 8 ? 1 : RBPS_NARROW_MIN_BLOCKS;
     template <class T, class P>
-    __global__ void __launch_bounds__(kMaxBlock, RBPS_NARROW_MIN_BLOCKS) k_flat_narrow(const Engine<T, P> E)
+    __global__ void __launch_bounds__(kMaxBlock, kNarrowBlocks<T>) k_flat_narrow(const Engine<T, P> E)
     {
         // the common-kind classes but box-box: [0, off(bb)) and [off(bb + 1), off(16))
         const uint32_t total = E.gcol[kGcolOff + kClassCommonEnd];
         const uint32_t bb0 = E.gcol[kGcolOff + kClassBoxBox], bb1 = E.gcol[kGcolOff + kClassBoxBox + 1];
         const uint32_t n = total - (bb1 - bb0);
-        const uint32_t per_warp = E.narrow_per_warp, lane = threadIdx.x & 31u;
-        const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-        const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
+        const uint32_t lane = threadIdx.x & 31u;
+        uint32_t per_warp = E.narrow_per_warp;
+        const uint32_t warp = narrow_warp(), n_warps = (gridDim.x * blockDim.x) >> 5;
+        if constexpr (sizeof(T) == 8)
+            per_warp = narrow_share(per_warp, n, n_warps);
         for (uint32_t base = warp * per_warp; base < n; base += n_warps * per_warp)
         {
             const uint32_t end = min(n, base + per_warp);
@@ -2360,13 +2382,15 @@ namespace rbps_gpu
     // The classes with another convex kind (ellipsoid, cylinder, cone, hull):
     // [off(16), off(25)).
     template <class T, class P>
-    __global__ void __launch_bounds__(kMaxBlock, RBPS_NARROW_MIN_BLOCKS) k_flat_narrow_other(const Engine<T, P> E)
+    __global__ void __launch_bounds__(kMaxBlock, kNarrowBlocks<T>) k_flat_narrow_other(const Engine<T, P> E)
     {
         const uint32_t o0 = E.gcol[kGcolOff + kClassCommonEnd], total = E.gcol[kGcolOff + kClassOtherEnd];
         const uint32_t n = total - o0;
-        const uint32_t per_warp = E.narrow_per_warp, lane = threadIdx.x & 31u;
-        const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-        const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
+        const uint32_t lane = threadIdx.x & 31u;
+        uint32_t per_warp = E.narrow_per_warp;
+        const uint32_t warp = narrow_warp(), n_warps = (gridDim.x * blockDim.x) >> 5;
+        if constexpr (sizeof(T) == 8)
+            per_warp = narrow_share(per_warp, n, n_warps);
         for (uint32_t base = warp * per_warp; base < n; base += n_warps * per_warp)
         {
             const uint32_t end = min(n, base + per_warp);
@@ -2410,13 +2434,15 @@ namespace rbps_gpu
     // The box-box class on its own: its SAT, clipping buffers and registers
     // stay out of the kernel that runs every other class.
     template <class T, class P>
-    __global__ void __launch_bounds__(kMaxBlock, RBPS_NARROW_MIN_BLOCKS) k_flat_narrow_boxbox(const Engine<T, P> E)
+    __global__ void __launch_bounds__(kMaxBlock, kNarrowBlocks<T>) k_flat_narrow_boxbox(const Engine<T, P> E)
     {
         const uint32_t bb0 = E.gcol[kGcolOff + kClassBoxBox], bb1 = E.gcol[kGcolOff + kClassBoxBox + 1];
         const uint32_t n = bb1 - bb0;
-        const uint32_t per_warp = E.narrow_per_warp, lane = threadIdx.x & 31u;
-        const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-        const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
+        const uint32_t lane = threadIdx.x & 31u;
+        uint32_t per_warp = E.narrow_per_warp;
+        const uint32_t warp = narrow_warp(), n_warps = (gridDim.x * blockDim.x) >> 5;
+        if constexpr (sizeof(T) == 8)
+            per_warp = narrow_share(per_warp, n, n_warps);
         for (uint32_t base = warp * per_warp; base < n; base += n_warps * per_warp)
         {
             const uint32_t end = min(n, base + per_warp);
