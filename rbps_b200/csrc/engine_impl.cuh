@@ -20,6 +20,8 @@
 // position solve (contacts, joint errors, joint rows), velocity update,
 // velocity solve (contacts, joint damping).
 #pragma once
+#include <initializer_list>
+
 #include "engine_types.cuh"
 #include "gjk.cuh"
 #include "team.cuh"
@@ -1135,21 +1137,35 @@ namespace rbps_gpu
         tm.sync();
     }
 
-    template <class T, class P>
-    __device__ uint32_t color_active(const Engine<T, P> &E, const GridTeam &tm, const WorldDev &W, const Scr<T, P> &S,
-                                     uint32_t n_cand, BlockShared &sh)
+    // Before it, the masks, counters and claims the rounds use are zeroed: by
+    // candidate (a warp a body's 64 claims) when they are few, else for every
+    // body.
+    template <class T, class P, class Team>
+    __device__ void color_rounds(const Engine<T, P> &E, const Team &tm, const WorldDev &W, const Scr<T, P> &S,
+                                 uint32_t n_act)
     {
         uint32_t *misc = S.misc;
-        for (uint32_t b = tm.rank(); b < W.n_bodies; b += tm.size())
-        {
-            S.bmask[b] = 0ull;
-            S.bprio[b] = 0ull;
-        }
-        for (uint32_t x = tm.rank(); x < W.n_bodies * 64u; x += tm.size())
-            S.claim[x] = 0ull;
-        for (uint32_t x = tm.rank(); x < kMaxColorRounds + 2 * 66; x += tm.size())
-            misc[kMiscCCount + x] = 0u;
-        const uint32_t n_act = compact_grid(tm, S, n_cand, sh);
+        auto clear = [&](uint32_t b) {
+            S.claim[(size_t)b * 64u + lane_id()] = 0ull;
+            S.claim[(size_t)b * 64u + 32u + lane_id()] = 0ull;
+            if (lane_id() == 0)
+            {
+                S.bmask[b] = 0ull;
+                S.bprio[b] = 0ull;
+            }
+        };
+        const uint32_t warp = tm.rank() >> 5, warps = tm.size() >> 5;
+        if (2u * n_act < W.n_bodies)
+            for (uint32_t q = warp; q < n_act; q += warps)
+            {
+                const Cand cd = S.cand[S.alist[q]];
+                clear(cd.ba);
+                clear(cd.bb);
+            }
+        else
+            for (uint32_t b = warp; b < W.n_bodies; b += warps)
+                clear(b);
+        tm.sync();
         const uint8_t *type = E.B.type + W.body_off;
         uint32_t round = 1;
         {
@@ -1273,7 +1289,33 @@ namespace rbps_gpu
         }
         tm.sync();
         color_overflow(E, tm, W, S);
-        return misc[kMiscFlags + 1];
+    }
+
+    // A grid barrier costs several block barriers, and the rounds take a
+    // dozen: up to kColorCtaMax contacts are coloured by CTA 0 alone, with
+    // the grid behind one barrier.  The colours are the same.  With that, the
+    // claims of contacting bodies alone zeroed (all of them are 33 MB in a
+    // 65,536-body world) and the phases of a step in one launch, the step of
+    // 20,625 chained capsules went from 3.77 to 3.48 ms, and the solves and
+    // the colouring of 65,536 bodies from 82 to 73 us a substep.
+    constexpr uint32_t kColorCtaMax = 1024;
+
+    template <class T, class P>
+    __device__ uint32_t color_active(const Engine<T, P> &E, const GridTeam &tm, const WorldDev &W, const Scr<T, P> &S,
+                                     uint32_t n_cand, BlockShared &sh)
+    {
+        for (uint32_t x = tm.rank(); x < kMaxColorRounds + 2 * 66; x += tm.size())
+            S.misc[kMiscCCount + x] = 0u;
+        const uint32_t n_act = compact_grid(tm, S, n_cand, sh);
+        if (n_act > kColorCtaMax)
+            color_rounds(E, tm, W, S, n_act);
+        else
+        {
+            if (blockIdx.x == 0)
+                color_rounds(E, BlockTeam(), W, S, n_act);
+            tm.sync();
+        }
+        return S.misc[kMiscFlags + 1];
     }
 
     // emit_contact (CollisionPipeline.cpp:59-104): a pair's manifold into
@@ -2092,9 +2134,12 @@ namespace rbps_gpu
         each_small_world(E.small_worlds, E.n_small, E.work_counter + ctr, [&](uint32_t w) { phase_stats(E, tm, w); });
     }
 
-    // One phase of one large world on the whole cooperative grid; the phases
-    // are separate launches so that the GJK pass can run between the
-    // narrowphase and the colouring, as it does for the small worlds.
+    // Phases of one large world on the whole cooperative grid, behind grid
+    // barriers: those of `first` (a nibble each, phase + 1, lowest first), then
+    // `again` those of `loop`, then those of `last`.  A launch and its drain
+    // cost more than a barrier: a step without a GJK pass is one launch, and
+    // a step with one has a launch between two passes.  Every phase has one
+    // call site, so it is the same code wherever it runs.
     // Resident 256-thread CTAs per SM of the cooperative grid, as for the
     // frame: capped at 128 registers (two CTAs), collision stress went from
     // 7.45 to 6.53 ms a step and joint-heavy from 5.53 to 5.12 ms (same box);
@@ -2104,18 +2149,42 @@ namespace rbps_gpu
 #endif
     template <class T, class P>
     __global__ void __launch_bounds__(kMaxBlock, RBPS_BIG_MIN_BLOCKS) k_big_phase(const Engine<T, P> E, uint32_t w,
-                                                                               int phase)
+                                                                               uint32_t first, uint32_t loop,
+                                                                               uint32_t again, uint32_t last)
     {
         __shared__ BlockShared sh;
         GridTeam tm;
-        switch (phase)
+        uint32_t seq = first;
+        for (;;)
         {
-        case kKFrame: phase_frame(E, tm, w, sh); break;
-        case kKNarrow: phase_narrow(E, tm, w); break;
-        case kKColor: phase_color_integrate(E, tm, w, sh); break;
-        case kKPosition: phase_position(E, tm, w); break;
-        case kKVelocity: phase_velocity(E, tm, w); break;
-        default: phase_stats(E, tm, w); break;
+            if (!seq && again)
+            {
+                seq = loop;
+                --again;
+            }
+            if (!seq)
+            {
+                seq = last;
+                last = 0;
+            }
+            if (!seq)
+                break;
+            switch ((int)(seq & 15u) - 1)
+            {
+            case kKFrame: phase_frame(E, tm, w, sh); break;
+            case kKNarrow: phase_narrow(E, tm, w); break;
+            case kKColor: phase_color_integrate(E, tm, w, sh); break;
+            case kKResetGjk:
+                // the queue for the narrowphase after the solves, whose
+                // barriers lie between
+                if (tm.leader())
+                    E.gjk_count[0] = E.gjk_count[1] = 0u;
+                break;
+            case kKPosition: phase_position(E, tm, w); break;
+            case kKVelocity: phase_velocity(E, tm, w); break;
+            default: phase_stats(E, tm, w); break;
+            }
+            seq >>= 4;
         }
     }
 
@@ -3235,43 +3304,48 @@ namespace rbps_gpu
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_substep<T, P, false, kSubstepBlocks<T>>, block, fl_smem);
     }
 
-    // Enqueues one step of one large world: 2 + 4 * substeps cooperative
-    // phase launches, plus the GJK pass after each narrowphase when the batch
-    // has one.  *launches receives the number of kernels enqueued.
+    // Enqueues one step of one large world: one cooperative launch, or with a
+    // GJK pass one before the first pass and one after each.  *launches
+    // receives the number of kernels enqueued.
     template <class T, class P>
     cudaError_t launch_step_big(const Engine<T, P> &e, uint32_t world, int grid, int block, cudaStream_t stream,
                                 long *launches)
     {
         Engine<T, P> ec = e;
-        int phase = 0;
-        void *args[] = {(void *)&ec, (void *)&world, (void *)&phase};
-        long n = 0;
-        auto run = [&](int ph) {
-            phase = ph;
-            ++n;
+        uint32_t first = 0, loop = 0, again = 0, last = 0;
+        void *args[] = {(void *)&ec, (void *)&world, (void *)&first, (void *)&loop, (void *)&again, (void *)&last};
+        auto phases = [](std::initializer_list<int> list) {
+            uint32_t seq = 0, at = 0;
+            for (int ph : list)
+                seq |= uint32_t(ph + 1) << (4 * at++);
+            return seq;
+        };
+        auto run = [&]() {
+            ++*launches;
             return cudaLaunchCooperativeKernel((const void *)k_big_phase<T, P>, dim3(grid), dim3(block), args, 0,
                                                stream);
         };
-        cudaError_t rc = run(kKFrame);
+        *launches = 0;
+        if (!e.gjk_list)
+        {
+            first = phases({kKFrame});
+            loop = phases({kKNarrow, kKColor, kKPosition, kKVelocity});
+            again = (uint32_t)e.substeps;
+            last = phases({kKStats});
+            return run();
+        }
+        cudaError_t rc = cudaMemsetAsync(e.gjk_count, 0, 8, stream);
+        first = phases({kKFrame, kKNarrow});
+        if (rc == cudaSuccess)
+            rc = run();
         for (int s = 0; s < e.substeps && rc == cudaSuccess; ++s)
         {
-            if (e.gjk_list && (rc = cudaMemsetAsync(e.gjk_count, 0, 8, stream)) != cudaSuccess)
+            if ((rc = launch_gjk(e, stream)) != cudaSuccess)
                 break;
-            if ((rc = run(kKNarrow)) != cudaSuccess)
-                break;
-            if (e.gjk_list)
-            {
-                if ((rc = launch_gjk(e, stream)) != cudaSuccess)
-                    break;
-                ++n;
-            }
-            if ((rc = run(kKColor)) != cudaSuccess || (rc = run(kKPosition)) != cudaSuccess ||
-                (rc = run(kKVelocity)) != cudaSuccess)
-                break;
+            ++*launches;
+            first = phases({kKColor, kKResetGjk, kKPosition, kKVelocity, s + 1 < e.substeps ? kKNarrow : kKStats});
+            rc = run();
         }
-        if (rc == cudaSuccess)
-            rc = run(kKStats);
-        *launches = n;
         return rc;
     }
 

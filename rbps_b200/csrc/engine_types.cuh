@@ -280,7 +280,7 @@ namespace rbps_gpu
     // Host entry points, instantiated per precision in engine_f64.cu /
     // engine_f32.cu.  They only enqueue work on `stream`.
     // Phases of a step: the frame and stats phases are kernels of the batched
-    // step; a large world runs all of them, one cooperative launch each.
+    // step; a large world runs all of them on the cooperative grid.
     enum : int
     {
         kKFrame = 0,
@@ -289,7 +289,8 @@ namespace rbps_gpu
         kKNarrow = 2,
         kKColor = 3,
         kKPosition = 4,
-        kKVelocity = 5
+        kKVelocity = 5,
+        kKResetGjk = 6
     };
     struct PhaseLaunch
     {
