@@ -14,6 +14,7 @@
 #include <cstring>
 #include <limits>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -319,6 +320,62 @@ struct HostHeightmap
     HmDesc d{};
 };
 
+// Page-locked staging of the state readback: two chunks of bodies and the
+// error words.  Locking its 1.7 MB takes a millisecond, more than a small
+// step, so a destroyed batch's goes to the next one: up to kKeep are kept,
+// the others unlocked.  A batch holds one from its first readback to its end
+// and gives it back after its streams have drained.
+constexpr uint32_t kStateChunk = 8192; // bodies
+
+struct StateStaging
+{
+    static constexpr size_t kSlot = (size_t)kStateChunk * 13; // doubles
+    static constexpr size_t kKeep = 8;
+
+    static double *take()
+    {
+        {
+            std::lock_guard<std::mutex> lock(mutex());
+            if (!kept().empty())
+            {
+                double *p = kept().back();
+                kept().pop_back();
+                return p;
+            }
+        }
+        void *p = nullptr;
+        return cudaHostAlloc(&p, (2 * kSlot + 8) * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped) ==
+                       cudaSuccess
+                   ? (double *)p
+                   : nullptr;
+    }
+    static void give(double *p)
+    {
+        {
+            std::lock_guard<std::mutex> lock(mutex());
+            if (kept().size() < kKeep)
+            {
+                kept().push_back(p);
+                return;
+            }
+        }
+        cudaFreeHost(p);
+    }
+
+private:
+    // never destroyed: a batch may outlive this file's statics
+    static std::mutex &mutex()
+    {
+        static std::mutex &m = *new std::mutex;
+        return m;
+    }
+    static std::vector<double *> &kept()
+    {
+        static std::vector<double *> &v = *new std::vector<double *>;
+        return v;
+    }
+};
+
 struct rbps_batch
 {
     rbps_batch_desc desc;
@@ -382,11 +439,11 @@ struct rbps_batch
     uint32_t gjk_cap = 0, gjk_slots = 0;
     PhaseLaunch phase{};      // grid / block of each phase kernel
     FlatLaunch flat{};        // flat colored pipeline
-    uint32_t *wcoff = nullptr, *gcol = nullptr, *sbodies = nullptr, *sjoints = nullptr, *sjcoff = nullptr;
+    uint32_t *wcoff = nullptr, *gcol = nullptr;
     uint2 *nlist = nullptr;
     uint4 *nglob = nullptr; // global collider / body indices beside nlist
     void **wcand = nullptr, **wcc = nullptr;
-    uint32_t n_sbodies = 0, n_sjoints = 0, n_sjcolors = 0, n_block_worlds = 0;
+    uint32_t n_block_worlds = 0;
     uint32_t smem_cap_block = 0, smem_cap_warp = 0, smem_cap_pair = 0, n_pair_worlds = 0;
     int grid_big = 0;
     uint32_t n_counters = 0;  // phase work counters per step
@@ -463,6 +520,13 @@ struct rbps_batch
     cudaEvent_t ev_force_ready[2] = {}, ev_force_free[2] = {}, ev_pose_ready[2] = {}, ev_out_free[2] = {};
     uint32_t io_slot = 0;
     bool io_async_ready = false;
+    // state readback (StateStaging)
+    double *state_host = nullptr;
+    cudaEvent_t ev_state[2] = {};
+    // rbps_batch_collide's device buffer, kept up to kCollideKeep bytes
+    static constexpr size_t kCollideKeep = size_t(64) << 20;
+    char *collide_dev = nullptr;
+    size_t collide_bytes = 0;
     // snapshot slots (rbps_batch_snapshot): one device buffer each, holding
     // the state arrays back to back
     std::vector<char *> snaps;
@@ -479,6 +543,12 @@ struct rbps_batch
             for (cudaEvent_t e : {ev_force_ready[k], ev_force_free[k], ev_pose_ready[k], ev_out_free[k]})
                 if (e)
                     cudaEventDestroy(e);
+        for (cudaEvent_t e : ev_state)
+            if (e)
+                cudaEventDestroy(e);
+        if (state_host)
+            StateStaging::give(state_host);
+        cudaFree(collide_dev);
         if (io_stream)
             cudaStreamDestroy(io_stream);
         if (io_out_stream)
@@ -875,12 +945,6 @@ namespace
         e.nglob = b->nglob;
         e.wcand = (Cand *const *)b->wcand;
         e.wcc = (CandContacts<T, P> *const *)b->wcc;
-        e.sbodies = b->sbodies;
-        e.n_sbodies = b->n_sbodies;
-        e.sjoints = b->sjoints;
-        e.sjcoff = b->sjcoff;
-        e.n_sjcolors = b->n_sjcolors;
-        e.n_sjoints = b->n_sjoints;
         e.small_worlds = b->small_list;
         e.n_small = (uint32_t)b->small_ids.size();
         e.n_block_worlds = b->n_block_worlds;
@@ -1487,8 +1551,6 @@ static int commit_typed(rbps_batch *b)
         const uint32_t ns = (uint32_t)b->small_ids.size();
         size_t cand_cap = 0;
         std::vector<void *> wcand(W, nullptr), wcc(W, nullptr);
-        std::vector<uint32_t> sbodies;
-        uint32_t max_jc = 0;
         for (uint32_t w : b->small_ids)
         {
             const WorldDev &d = b->wdev[w];
@@ -1496,35 +1558,19 @@ static int commit_typed(rbps_batch *b)
             wcand[w] = b->scratch + d.scr_off + L.cand;
             wcc[w] = b->scratch + d.scr_off + L.cc;
             cand_cap += (size_t)d.pair_cap + 1 + d.n_pc;
-            for (uint32_t k = 0; k < d.n_bodies; ++k)
-                sbodies.push_back(d.body_off + k);
-            max_jc = std::max(max_jc, d.n_jcolors);
         }
-        std::vector<uint32_t> sjoints, sjcoff(1, 0);
-        for (uint32_t jc = 0; jc < max_jc; ++jc)
-        {
-            for (uint32_t w : b->small_ids)
-            {
-                const WorldDev &d = b->wdev[w];
-                if (jc >= d.n_jcolors)
-                    continue;
-                for (uint32_t k = joffs[w][jc]; k < joffs[w][jc + 1]; ++k)
-                    sjoints.push_back(d.joint_off + jorders[w][k]);
-            }
-            sjcoff.push_back((uint32_t)sjoints.size());
-        }
-        b->n_sbodies = (uint32_t)sbodies.size();
-        b->n_sjoints = (uint32_t)sjoints.size();
-        b->n_sjcolors = max_jc;
-        if ((rc = b->alloc((void **)&b->wcoff, 4 * ((size_t)ns + 1))) ||
-            (rc = b->alloc((void **)&b->gcol, 4 * (size_t)kGcolWords)) ||
-            (rc = b->alloc((void **)&b->nlist, sizeof(uint2) * std::max<size_t>(cand_cap, 1))) ||
-            (rc = b->alloc((void **)&b->nglob, sizeof(uint4) * std::max<size_t>(cand_cap, 1))) ||
-            (rc = b->upload(&b->wcand, wcand)) || (rc = b->upload(&b->wcc, wcc)) ||
-            (rc = b->upload(&b->sbodies, sbodies)) || (rc = b->upload(&b->sjoints, sjoints)) ||
-            (rc = b->upload(&b->sjcoff, sjcoff)))
+        // one allocation for the class-sorted list (nlist beside nglob) and
+        // the words (gcol, wcoff), one for the worlds' pointers
+        const size_t list = std::max<size_t>(cand_cap, 1);
+        wcand.insert(wcand.end(), wcc.begin(), wcc.end());
+        if ((rc = b->alloc((void **)&b->nglob,
+                           (sizeof(uint4) + sizeof(uint2)) * list + 4 * (kGcolWords + (size_t)ns + 1))) ||
+            (rc = b->upload(&b->wcand, wcand)))
             return rc;
-        CU(cudaMemset(b->gcol, 0, 4 * (size_t)kGcolWords));
+        b->nlist = reinterpret_cast<uint2 *>(b->nglob + list);
+        b->gcol = reinterpret_cast<uint32_t *>(b->nlist + list);
+        b->wcoff = b->gcol + kGcolWords;
+        b->wcc = b->wcand + W;
         int per_sm = 0;
         CU(occupancy_flat<T, P>(0, kMaxBlockHost, &per_sm, 0));
         b->flat.grid_narrow = std::max(1, per_sm) * b->sm_count;
@@ -1536,10 +1582,6 @@ static int commit_typed(rbps_batch *b)
         b->flat.sm_count = b->sm_count;
         if ((rc = set_team_split<T, P>(b, kBlockTeamBodies, kPairTeamBodies)))
             return rc;
-        // side stream + events for the parallel narrowphase kernels
-        CU(cudaStreamCreateWithFlags(&b->flat.side, cudaStreamNonBlocking));
-        CU(cudaEventCreateWithFlags(&b->flat.fork, cudaEventDisableTiming));
-        CU(cudaEventCreateWithFlags(&b->flat.join, cudaEventDisableTiming));
     }
     for (const auto &w : b->worlds)
         for (const auto &c : w.colliders)
@@ -1566,14 +1608,16 @@ static int commit_typed(rbps_batch *b)
             // the GJK pass: one warp per queued pair, its polytope and
             // clipping buffers in shared memory; as many CTAs as stay resident
             CU(prepare_gjk<T, P>(b->sm_count, &b->gjk_slots));
-            if ((rc = b->alloc((void **)&b->gjk_list, sizeof(uint2) * cap)) ||
-                (rc = b->alloc((void **)&b->gjk_count, 64)))
+            if ((rc = b->alloc((void **)&b->gjk_count, 64 + sizeof(uint2) * cap)))
                 return rc;
+            b->gjk_list = reinterpret_cast<uint2 *>(b->gjk_count + 16);
         }
     }
-    if ((rc = b->alloc((void **)&b->work_counter, std::max<size_t>(64, 4 * (size_t)b->n_counters))) || (rc = b->alloc((void **)&b->error_d, 64)) ||
-        (rc = b->alloc((void **)&b->stats_d, sizeof(WorldStats) * W)))
+    static_assert(sizeof(WorldStats) % 16 == 0, "WorldStats rows after the counters and the error words");
+    if ((rc = b->alloc((void **)&b->work_counter, 128 + sizeof(WorldStats) * W)))
         return rc;
+    b->error_d = reinterpret_cast<int *>(b->work_counter + 16);
+    b->stats_d = reinterpret_cast<WorldStats *>(b->work_counter + 32);
     if ((rc = b->upload(&b->worlds_d, b->wdev)))
         return rc;
     return RBPS_OK;
@@ -1710,6 +1754,15 @@ static void capture_step(rbps_batch *b, const Engine<T, P> &e, int key)
 template <class T, class P>
 static int step_typed(rbps_batch *b, int n)
 {
+    // side stream + events for the parallel narrowphase kernels, with the
+    // first step: a batch that only answers queries has no use for them
+    if (!b->small_ids.empty() && n > 0 && !b->flat.side)
+    {
+        for (cudaEvent_t *ev : {&b->flat.fork, &b->flat.join})
+            if (!*ev)
+                CU(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+        CU(cudaStreamCreateWithFlags(&b->flat.side, cudaStreamNonBlocking));
+    }
     Engine<T, P> e = make_engine<T, P>(b);
     const int key = (b->dump ? 1 : 0) | (e.prof ? 2 : 0) | (e.check_state ? 4 : 0);
     if (b->graph_ok && n > 0 && (!b->graph_exec || b->graph_key != key))
@@ -1802,44 +1855,60 @@ extern "C" int rbps_batch_synchronize(rbps_batch *b)
 }
 
 // ------------------------------------------------------------ readback
+// The state in doubles, kStateChunk bodies at a time: the device converts a
+// chunk straight into page-locked memory, and the host moves it on while the
+// next one is under way.  Reading the device's arrays into fresh vectors and
+// converting there cost more than the copies (65,536 bodies: 1.6 ms, 0.8 so),
+// and four synchronous copies cost a small world 100 us where one launch
+// does.  The error word comes with the first chunk; on a device error nothing
+// is written.  Waits for the batch's stream.
+static int check_device_error(rbps_batch *b);
+
 template <class T, class P>
 static int get_state_typed(rbps_batch *b, uint32_t first, uint32_t n, const rbps_state_view *v)
 {
-    std::vector<V4<P>> pos(n);
-    std::vector<Q4<T>> rot(n);
-    std::vector<V4<T>> lin(n), ang(n);
-    if (v->position)
-        CU(cudaMemcpy(pos.data(), (V4<P> *)b->pos + first, n * sizeof(V4<P>), cudaMemcpyDeviceToHost));
-    if (v->orientation)
-        CU(cudaMemcpy(rot.data(), (Q4<T> *)b->rot + first, n * sizeof(Q4<T>), cudaMemcpyDeviceToHost));
-    if (v->linear_velocity)
-        CU(cudaMemcpy(lin.data(), (V4<T> *)b->lin + first, n * sizeof(V4<T>), cudaMemcpyDeviceToHost));
-    if (v->angular_velocity)
-        CU(cudaMemcpy(ang.data(), (V4<T> *)b->ang + first, n * sizeof(V4<T>), cudaMemcpyDeviceToHost));
-    for (uint32_t i = 0; i < n; ++i)
+    constexpr uint32_t kWidth[4] = {3, 4, 3, 3};
+    double *const to[4] = {v->position, v->orientation, v->linear_velocity, v->angular_velocity};
+    uint32_t width = 0, mask = 0;
+    for (int f = 0; f < 4; ++f)
+        if (to[f])
+        {
+            width += kWidth[f];
+            mask |= 1u << f;
+        }
+    if (!b->state_host && !(b->state_host = StateStaging::take()))
+        return fail(RBPS_ERR_CUDA, "rbps_batch_get_state: no page-locked memory");
+    for (cudaEvent_t &ev : b->ev_state)
+        if (!ev)
+            CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    const Engine<T, P> e = make_engine<T, P>(b);
+    const uint32_t cap = kStateChunk, chunks = n && width ? (n + cap - 1) / cap : 0;
+    int *err = reinterpret_cast<int *>(b->state_host + 2 * StateStaging::kSlot);
+    auto issue = [&](uint32_t c) {
+        const uint32_t i0 = c * cap, m = chunks ? std::min(cap, n - i0) : 0;
+        const cudaError_t rc = launch_state_out<T, P>(e, b->state_host + (c & 1) * StateStaging::kSlot, first + i0, m,
+                                                      mask, c ? nullptr : err, b->stream);
+        return rc == cudaSuccess ? cudaEventRecord(b->ev_state[c & 1], b->stream) : rc;
+    };
+    CU(issue(0));
+    for (uint32_t c = 0; c < std::max(chunks, 1u); ++c)
     {
-        if (v->position)
+        if (c + 1 < chunks)
+            CU(issue(c + 1));
+        CU(cudaEventSynchronize(b->ev_state[c & 1]));
+        if (c == 0 && err[0])
         {
-            const double *o = b->origin_of_body(first + i);
-            v->position[3 * i] = o[0] + double(pos[i].x);
-            v->position[3 * i + 1] = o[1] + double(pos[i].y);
-            v->position[3 * i + 2] = o[2] + double(pos[i].z);
+            CU(cudaStreamSynchronize(b->stream));
+            return check_device_error(b);
         }
-        if (v->orientation)
-        {
-            v->orientation[4 * i] = rot[i].w; v->orientation[4 * i + 1] = rot[i].x;
-            v->orientation[4 * i + 2] = rot[i].y; v->orientation[4 * i + 3] = rot[i].z;
-        }
-        if (v->linear_velocity)
-        {
-            v->linear_velocity[3 * i] = lin[i].x; v->linear_velocity[3 * i + 1] = lin[i].y;
-            v->linear_velocity[3 * i + 2] = lin[i].z;
-        }
-        if (v->angular_velocity)
-        {
-            v->angular_velocity[3 * i] = ang[i].x; v->angular_velocity[3 * i + 1] = ang[i].y;
-            v->angular_velocity[3 * i + 2] = ang[i].z;
-        }
+        const uint32_t i0 = c * cap, m = std::min(cap, n - i0);
+        const double *from = b->state_host + (c & 1) * StateStaging::kSlot;
+        for (int f = 0; f < 4 && chunks; ++f)
+            if (to[f])
+            {
+                std::memcpy(to[f] + (size_t)i0 * kWidth[f], from, (size_t)m * kWidth[f] * 8);
+                from += (size_t)m * kWidth[f];
+            }
     }
     return RBPS_OK;
 }
@@ -1893,11 +1962,12 @@ static int ready(rbps_batch *b, const char *who)
 
 extern "C" int rbps_batch_get_state(rbps_batch *b, uint32_t world, const rbps_state_view *v)
 {
-    int rc = ready(b, "rbps_batch_get_state");
-    if (rc)
-        return rc;
-    if (!v || world >= b->wdev.size())
-        return fail(RBPS_ERR_INVALID, "rbps_batch_get_state: bad world or view");
+    if (!b || !b->committed || !v || world >= b->wdev.size())
+    {
+        const int rc = ready(b, "rbps_batch_get_state");
+        return rc ? rc : fail(RBPS_ERR_INVALID, "rbps_batch_get_state: bad world or view");
+    }
+    CU(cudaSetDevice(b->desc.device));
     return DISPATCH_PREC(b, get_state_typed, b, b->wdev[world].body_off, b->wdev[world].n_bodies, v);
 }
 
@@ -1913,11 +1983,12 @@ extern "C" int rbps_batch_set_state(rbps_batch *b, uint32_t world, const rbps_st
 
 extern "C" int rbps_batch_get_state_all(rbps_batch *b, const rbps_state_view *v)
 {
-    int rc = ready(b, "rbps_batch_get_state_all");
-    if (rc)
-        return rc;
-    if (!v)
-        return fail(RBPS_ERR_INVALID, "null view");
+    if (!b || !b->committed || !v)
+    {
+        const int rc = ready(b, "rbps_batch_get_state_all");
+        return rc ? rc : fail(RBPS_ERR_INVALID, "null view");
+    }
+    CU(cudaSetDevice(b->desc.device));
     return DISPATCH_PREC(b, get_state_typed, b, 0u, b->n_bodies_all, v);
 }
 
@@ -2258,13 +2329,17 @@ static int collide_typed(rbps_batch *b, uint32_t n, const std::vector<ShapeDev> 
     HullSetDev hs{b->hull_verts, b->hull_voff, b->hull_aabb, b->hull_desc, b->hull_u32, b->hull_pn, b->hm_heights,
                   b->hm_desc, b->mesh_desc, b->mesh_v, b->mesh_i, b->mesh_n};
     const size_t shape_bytes = (size_t)n * sizeof(ShapeDev), tf_bytes = (size_t)n * 7 * sizeof(double);
-    bool gjk = false;
-    for (uint32_t i = 0; i < n && !gjk; ++i)
-        gjk = (gjk_kind(sa[i].kind) || gjk_kind(sb[i].kind)) && sa[i].kind != kPlane && sb[i].kind != kPlane;
-    (void)gjk; // one warp per pair, GJK workspaces in shared memory
-    char *d = nullptr;
     const size_t total = 2 * shape_bytes + 2 * tf_bytes + (size_t)n * sizeof(CollideOut);
-    CU(cudaMalloc(&d, total));
+    // cudaMalloc and cudaFree took longer than a few thousand pairs
+    if (total > b->collide_bytes)
+    {
+        cudaFree(b->collide_dev);
+        b->collide_dev = nullptr;
+        b->collide_bytes = 0;
+        CU(cudaMalloc(&b->collide_dev, total));
+        b->collide_bytes = total;
+    }
+    char *d = b->collide_dev;
     ShapeDev *dsa = (ShapeDev *)d, *dsb = (ShapeDev *)(d + shape_bytes);
     double *dta = (double *)(d + 2 * shape_bytes), *dtb = (double *)(d + 2 * shape_bytes + tf_bytes);
     CollideOut *dout = (CollideOut *)(d + 2 * shape_bytes + 2 * tf_bytes);
@@ -2281,7 +2356,12 @@ static int collide_typed(rbps_batch *b, uint32_t n, const std::vector<ShapeDev> 
         e = cudaMemcpyAsync(out, dout, (size_t)n * sizeof(CollideOut), cudaMemcpyDeviceToHost, b->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(b->stream);
-    cudaFree(d);
+    if (b->collide_bytes > rbps_batch::kCollideKeep)
+    {
+        cudaFree(b->collide_dev);
+        b->collide_dev = nullptr;
+        b->collide_bytes = 0;
+    }
     if (e != cudaSuccess)
         return fail(RBPS_ERR_CUDA, "rbps_batch_collide: %s", cudaGetErrorString(e));
     return b->committed ? check_device_error(b) : RBPS_OK;

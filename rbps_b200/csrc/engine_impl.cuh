@@ -3377,6 +3377,8 @@ namespace rbps_gpu
     template cudaError_t rbps_gpu::occupancy_big<T, P>(int, int *);                                               \
     template cudaError_t rbps_gpu::launch_debug_broadphase<T, P>(const rbps_gpu::Engine<T, P> &, uint32_t, int,    \
                                                                  uint32_t *, cudaStream_t);                         \
+    template cudaError_t rbps_gpu::launch_state_out<T, P>(const rbps_gpu::Engine<T, P> &, double *, uint32_t,      \
+                                                          uint32_t, uint32_t, int *, cudaStream_t);               \
     template cudaError_t rbps_gpu::launch_io<T, P>(const rbps_gpu::Engine<T, P> &, int, double *, double *,       \
                                                    uint32_t, int, cudaStream_t);
 
@@ -3412,6 +3414,46 @@ namespace rbps_gpu
             rot[4 * i + 2] = double(q.y);
             rot[4 * i + 3] = double(q.z);
         }
+    }
+
+    // Each field is n rows of its width: consecutive threads write
+    // consecutive doubles, so the rows go out whole.
+    template <class T, class P>
+    __global__ void k_state_out(const Engine<T, P> E, double *out, uint32_t first, uint32_t n, uint32_t mask,
+                                int *err_out)
+    {
+        if (err_out && blockIdx.x == 0 && threadIdx.x < 4)
+            err_out[threadIdx.x] = E.error[threadIdx.x];
+        for (uint32_t f = 0; f < 4; ++f)
+        {
+            if (!(mask >> f & 1u))
+                continue;
+            const uint32_t w = f == 1 ? 4u : 3u;
+            for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < w * n; x += gridDim.x * blockDim.x)
+            {
+                const uint32_t i = first + x / w, k = x % w;
+                double v;
+                if (f == 0)
+                {
+                    const double o = E.origin ? E.origin[3 * (size_t)E.body_world[i] + k] : 0.0;
+                    v = o + double(reinterpret_cast<const P *>(E.B.pos + i)[k]);
+                }
+                else
+                    v = double(f == 1   ? reinterpret_cast<const T *>(E.B.rot + i)[k]
+                               : f == 2 ? reinterpret_cast<const T *>(E.B.lin + i)[k]
+                                        : reinterpret_cast<const T *>(E.B.ang + i)[k]);
+                out[x] = v;
+            }
+            out += (size_t)w * n;
+        }
+    }
+
+    template <class T, class P>
+    cudaError_t launch_state_out(const Engine<T, P> &e, double *out, uint32_t first, uint32_t n, uint32_t mask,
+                                 int *err_out, cudaStream_t stream)
+    {
+        k_state_out<T, P><<<n / 256 + 1, 256, 0, stream>>>(e, out, first, n, mask, err_out);
+        return cudaGetLastError();
     }
 
     template <class T, class P>

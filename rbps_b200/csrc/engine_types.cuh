@@ -265,11 +265,6 @@ namespace rbps_gpu
         uint4 *nglob;                  // beside each entry: global colliders a, b and bodies a, b
         Cand *const *wcand;            // per world: its candidate list
         CandContacts<T, P> *const *wcc; // per world: its contact manifolds
-        const uint32_t *sbodies;       // bodies of the small worlds
-        uint32_t n_sbodies;
-        const uint32_t *sjoints;       // joints of the small worlds grouped by joint colour
-        const uint32_t *sjcoff;        // n_sjcolors + 1 offsets into sjoints
-        uint32_t n_sjcolors, n_sjoints;
     };
 
     // gcol layout (u32 words): per shape-pair class [0, 64) counts, [64, 128)
@@ -334,6 +329,12 @@ namespace rbps_gpu
     template <class T, class P>
     cudaError_t launch_io(const Engine<T, P> &e, int dir, double *a, double *b, uint32_t n, int grid,
                           cudaStream_t stream);
+    // bodies [first, first + n) in doubles, the fields of `mask` one after
+    // another: position (bit 0), orientation wxyz, linear, angular velocity;
+    // and, unless null, the batch's four error words
+    template <class T, class P>
+    cudaError_t launch_state_out(const Engine<T, P> &e, double *out, uint32_t first, uint32_t n, uint32_t mask,
+                                 int *err_out, cudaStream_t stream);
     // Output of one device narrowphase test; the layout of rbps_manifold.
     struct CollideOut
     {
