@@ -268,6 +268,82 @@ namespace rbps_gpu
             tm.sync();
         }
     }
+    // The same on one CTA, for fewer than 65,536 pairs: a thread keeps a run
+    // of consecutive pairs, counts its 4-bit digits in a column of its own
+    // (sh.wdig as 16-bit counters, digit-major, so one scan over all of them
+    // ranks the pairs stably), and places its run.  A pass costs one block
+    // scan however many pairs there are, where the tiles above cost six
+    // barriers and two scans for every 256 of them (a static query of 1,999
+    // objects: 300 us with the tiles, 236 so).  A digit that all keys share
+    // is skipped.
+    static __device__ __noinline__ void team_radix_sort(const BlockTeam &tm, uint32_t *keys, uint32_t *vals, uint32_t *kt,
+                                                        uint32_t *vt, uint32_t n, int bits, uint32_t *counts,
+                                                        uint32_t *tile_sums, BlockShared &sh)
+    {
+        if (n >= 65536u)
+        {
+            team_radix_sort<BlockTeam>(tm, keys, vals, kt, vt, n, bits, counts, tile_sums, sh);
+            return;
+        }
+        if (n <= 1)
+            return;
+        uint16_t *cnt = reinterpret_cast<uint16_t *>(sh.wdig);
+        const uint32_t B = blockDim.x, t = threadIdx.x;
+        const uint32_t per = (n + B - 1) / B;
+        const uint32_t i0 = min(n, t * per), i1 = min(n, i0 + per);
+        uint32_t *a_k = keys, *a_v = vals, *b_k = kt, *b_v = vt;
+        for (int shift = 0; shift < bits; shift += 4)
+        {
+            for (uint32_t d = 0; d < 16; ++d)
+                cnt[d * B + t] = 0;
+            for (uint32_t i = i0; i < i1; ++i)
+                ++cnt[((a_k[i] >> shift) & 15u) * B + t];
+            __syncthreads();
+            uint32_t sum = 0;
+            for (uint32_t x = 16 * t; x < 16 * t + 16; ++x)
+                sum += cnt[x];
+            uint32_t total;
+            uint32_t run = block_excl_scan(sum, sh, &total);
+            for (uint32_t x = 16 * t; x < 16 * t + 16; ++x)
+            {
+                const uint32_t c = cnt[x];
+                cnt[x] = (uint16_t)run;
+                run += c;
+            }
+            __syncthreads();
+            bool one = false; // a digit that all keys share
+            for (uint32_t d = 0; d < 16; ++d)
+                one = one || (d + 1 < 16 ? cnt[(d + 1) * B] : n) - cnt[d * B] == n;
+            __syncthreads();
+            if (one)
+                continue;
+            for (uint32_t i = i0; i < i1; ++i)
+            {
+                const uint32_t key = a_k[i], c = ((key >> shift) & 15u) * B + t;
+                const uint32_t dst = cnt[c];
+                cnt[c] = (uint16_t)(dst + 1);
+                b_k[dst] = key;
+                b_v[dst] = a_v[i];
+            }
+            __syncthreads();
+            uint32_t *x = a_k;
+            a_k = b_k;
+            b_k = x;
+            x = a_v;
+            a_v = b_v;
+            b_v = x;
+        }
+        if (a_k != keys)
+        {
+            for (uint32_t i = t; i < n; i += B)
+            {
+                keys[i] = a_k[i];
+                vals[i] = a_v[i];
+            }
+            __syncthreads();
+        }
+    }
+
     // A sort staged in shared memory: a CTA team with `smem` (kSmemSortWords
     // words) and at least 128 threads copies up to kSmemSortMax (key, value)
     // pairs in, runs the same stable radix sort on the shared copies and
