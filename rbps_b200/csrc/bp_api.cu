@@ -277,7 +277,7 @@ extern "C" int rbps_bp_update(rbps_bp *bp)
             cudaMemcpy(bp->d_id, bp->order.data(), nep * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
             cudaMemset(bp->d_err, 0, 4) != cudaSuccess)
             return bfail(RBPS_ERR_CUDA, "rbps_bp_update: upload failed");
-        const int grid = (int)std::max<size_t>(1, std::min<size_t>((nep + 1023) / 1024, (size_t)bp->occ * bp->sms));
+        const int grid = (int)std::max<size_t>(1, std::min<size_t>((nep + 255) / 256, (size_t)bp->occ * bp->sms));
         uint32_t cap = (uint32_t)bp->cap_pairs;
         uint32_t id_limit = (uint32_t)(2 * no);
         void *args[] = {&bp->d_fat, &bp->d_key, &bp->d_id, &bp->d_pos, (void *)&nbp, &id_limit, &cap, &bp->d_err,
