@@ -984,8 +984,16 @@ namespace
 
     constexpr uint32_t kSmallWorldBodies = kGridWorldBodies; // larger worlds step on the cooperative grid
     constexpr int kMaxBlockHost = 256; // block of the flat kernels (their __launch_bounds__)
-    constexpr uint32_t kBlockTeamBodies = 256; // colored batches: worlds this large step on a whole CTA
-    constexpr uint32_t kPairTeamBodies = 96;   // ... and worlds this large on half a CTA
+    // The default team split: worlds of kBlockTeamBodies or more step on a
+    // whole CTA, of kPairTeamBodies or more on half a CTA, others on a warp.
+    // Up to kFewWorldsPerSm worlds an SM every CTA is resident at once, and a
+    // smaller world has no one to leave the other warps to: CTAs from
+    // kPairTeamBodies on.  4,096 uneven worlds: 5.39 ms a step at 256 / 96,
+    // 5.18 at 192 / 64; 256 towers of 65 bodies: 1.68 ms on warps, 1.53 on
+    // CTAs; 61 uneven worlds: 0.82 either way.
+    constexpr uint32_t kBlockTeamBodies = 192;
+    constexpr uint32_t kPairTeamBodies = 64;
+    constexpr uint32_t kFewWorldsPerSm = 3;
     constexpr size_t kSmemWorldsMax = 226 * 1024; // bytes of world copies a CTA can open (227 KB less the scan words)
     constexpr uint32_t kSmemBodiesMax = 1024;   // bodies a CTA world keeps in shared memory (137 KB in FP32)
 } // namespace
@@ -1580,7 +1588,8 @@ static int commit_typed(rbps_batch *b)
         b->flat.grid_sort = std::max(1, per_sm) * b->sm_count;
         b->flat.block_solve = 128;
         b->flat.sm_count = b->sm_count;
-        if ((rc = set_team_split<T, P>(b, kBlockTeamBodies, kPairTeamBodies)))
+        const bool few = ns <= kFewWorldsPerSm * (uint32_t)b->sm_count;
+        if ((rc = set_team_split<T, P>(b, few ? kPairTeamBodies : kBlockTeamBodies, kPairTeamBodies)))
             return rc;
     }
     for (const auto &w : b->worlds)
