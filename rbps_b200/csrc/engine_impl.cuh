@@ -2008,6 +2008,32 @@ namespace rbps_gpu
                 tm.sync();
             }
         }
+        // In list order a chain's damping is a level a joint.  A joint that
+        // does nothing to the velocities as they are leaves them so for the
+        // next, so when none does, the levels are passed over: 12 of them were
+        // 7 us of a 13 us velocity solve in worlds without damping.  (Double
+        // only: float would contract its rows otherwise.)
+        if constexpr (Ref && kSplitPairs<T>)
+            if (W.n_jcolors > 2)
+            {
+                if (tm.leader())
+                    S.misc[kMiscFlags] = 0u;
+                tm.sync();
+                for (uint32_t j = tm.rank(); j < W.n_joints; j += tm.size())
+                {
+                    Joint<T> jt = E.joints[W.joint_off + j];
+                    jt.b1 -= shift;
+                    jt.b2 -= shift;
+                    if (joint_damps(B, jt, E.h))
+                        S.misc[kMiscFlags] = 1u;
+                }
+                tm.sync();
+                if (S.misc[kMiscFlags] == 0u)
+                {
+                    clk.mark(kPhVelSolve);
+                    return;
+                }
+            }
         const uint32_t *jco = E.jcolor_off + W.jc_off;
         for (uint32_t jc = 0; jc < W.n_jcolors; ++jc)
         {

@@ -950,6 +950,17 @@ namespace rbps_gpu
         store_pose(B, i, X);
     }
 
+    // Whether joint_damping does anything to the joint's bodies as they are.
+    template <class T, class P>
+    __device__ __forceinline__ bool joint_damps(const Bodies<T, P> &B, const Joint<T> &j, T h)
+    {
+        if (j.type != kRevolute && j.type != kPrismatic)
+            return false;
+        const V4<T> *v = j.type == kRevolute ? B.ang : B.lin;
+        const vec3<T> d = (v3(v[j.b2]) - v3(v[j.b1])) * rmin(j.damping * h, T(1.0));
+        return !(length_sq(d) < T(kEpsilon));
+    }
+
     // apply_{prismatic,revolute}_joint_damping (Joint.cpp:184-220)
     template <class T, class P>
     __device__ __noinline__ void joint_damping(const Bodies<T, P> &B, const Joint<T> &j, T h)
