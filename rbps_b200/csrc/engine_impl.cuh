@@ -14,11 +14,10 @@
 //      order bp_sweep emits them (BroadPhase.cpp:104-152)
 //   4. narrowphase candidates: filtered SAP pairs, then the static
 //      plane-vs-collider list (CollisionPipeline.cpp:110-198)
-//   5. colored mode only: Jones-Plassmann colouring of the candidates by
-//      shared dynamic bodies
-// Substeps (World.hpp:203-211): narrowphase + contact emission, integrate,
-// position solve (contacts, joint errors, joint rows), velocity update,
-// velocity solve (contacts, joint damping).
+// Substeps (World.hpp:203-211): narrowphase + contact emission, the order of
+// the contacting candidates (colours, or in reference order levels),
+// integrate, position solve (contacts, joint errors, joint rows), velocity
+// update, velocity solve (contacts, joint damping).
 #pragma once
 #include <initializer_list>
 
@@ -390,6 +389,8 @@ namespace rbps_gpu
             mine += opens(ep_id[i]) ? 1u : 0u;
         uint32_t n_open;
         uint32_t run = block_excl_scan(mine, sh, &n_open);
+        if (n_open > nep / 2) // half the endpoints open: a corrupt list, left to sweep_runs to report
+            return ~0u;
         // position | run end << 16, first slots and fill counts per opening
         // endpoint; then, in what is left, the extents in the first half and
         // the list in the second, and the grouped list over the extents
@@ -546,16 +547,19 @@ namespace rbps_gpu
             S.misc[kMiscFlags + 4] = 0u; // pairs found
         }
         tm.sync();
-        const uint32_t n_open = team_excl_scan(tm, S.cnt, S.cnt, nep, S.tile_sums, sh);
+        const uint32_t n_found = team_excl_scan(tm, S.cnt, S.cnt, nep, S.tile_sums, sh);
+        const uint32_t n_open = min(n_found, nep / 2); // what yz holds
+        if (n_found > n_open && tm.leader())
+            set_error_at(error, kErrInternal, 1, n_found);
         for (uint32_t i = tm.rank(); i < nep; i += tm.size())
         {
             const uint32_t id = ep_id[i];
-            if ((id & 1u) || id >= id_limit)
+            if ((id & 1u) || id >= id_limit || S.cnt[i] >= n_open)
                 continue;
             const uint32_t k = S.cnt[i], end = ep_pos[id + 1];
             const FatBox f = fat[id >> 1];
             o_pos[k] = i;
-            o_end[k] = end < nep ? S.cnt[end] : n_open;
+            o_end[k] = min(end < nep ? S.cnt[end] : n_open, n_open);
             yz[k] = make_float4(__double2float_rd(f.mn[1]), __double2float_ru(f.mx[1]), __double2float_rd(f.mn[2]),
                                 __double2float_ru(f.mx[2]));
         }
