@@ -1076,7 +1076,9 @@ namespace rbps_gpu
     // solves can relax it colour by colour (kMiscC2Off) instead of on one
     // thread; entry 64 keeps what still does not fit.  The bucket comes
     // after every first-level colour, so the Gauss-Seidel order stays a
-    // sequence of conflict-free sets.
+    // sequence of conflict-free sets.  It is handed over in list order and
+    // every candidate keeps its rank within its colour, so the order is the
+    // same in every run.
     template <class T, class P, class Team>
     __device__ void color_overflow(const Engine<T, P> &E, const Team &tm, const WorldDev &W, const Scr<T, P> &S)
     {
@@ -1090,7 +1092,7 @@ namespace rbps_gpu
             for (uint32_t b = tm.rank(); b < W.n_bodies; b += tm.size())
                 S.bprio[b] = 0ull;
             for (uint32_t q = s0 + tm.rank(); q < s1; q += tm.size())
-                S.alist[q - s0] = S.corder[q];
+                S.alist[q - s0] = S.loff[q - s0];
         }
         tm.sync();
         if (tm.leader())
@@ -1128,25 +1130,23 @@ namespace rbps_gpu
                             if (db[k])
                                 S.bprio[cd[k].bb] |= bit;
                         }
-                        S.act[cs[k]] = col;
+                        S.act[cs[k]] = cnt[col] << 7 | col;
                         cnt[col] += 1u;
                     }
             }
             uint32_t run = s0;
             for (uint32_t k = 0; k <= kColorSerial; ++k)
             {
-                const uint32_t n = cnt[k];
                 off[k] = run;
-                cnt[k] = run; // fill cursor
-                run += n;
+                run += cnt[k];
             }
             off[kColorSerial + 1] = run;
         }
         tm.sync();
         for (uint32_t q = tm.rank(); q < s1 - s0; q += tm.size())
         {
-            const uint32_t c = S.alist[q];
-            S.corder[atomicAdd(&cnt[S.act[c]], 1u)] = c;
+            const uint32_t c = S.alist[q], a = S.act[c];
+            S.corder[off[a & 127u] + (a >> 7)] = c;
         }
         tm.sync();
     }
@@ -1156,7 +1156,7 @@ namespace rbps_gpu
     // body.
     template <class T, class P, class Team>
     __device__ void color_rounds(const Engine<T, P> &E, const Team &tm, const WorldDev &W, const Scr<T, P> &S,
-                                 uint32_t n_act)
+                                 uint32_t n_act, BlockShared &sh)
     {
         uint32_t *misc = S.misc;
         auto clear = [&](uint32_t b) {
@@ -1297,9 +1297,19 @@ namespace rbps_gpu
         tm.sync();
         for (uint32_t q = tm.rank(); q < n_act; q += tm.size())
         {
-            const uint32_t c = S.alist[q];
-            const uint32_t slot = atomicAdd(&misc[kMiscCCount + S.color[c]], 1u);
-            S.corder[slot] = c;
+            const uint32_t c = S.alist[q], col = S.color[c];
+            if (col != kColorSerial)
+                S.corder[atomicAdd(&misc[kMiscCCount + col], 1u)] = c;
+        }
+        if (misc[kMiscCOff + kColorSerial + 1] > misc[kMiscCOff + kColorSerial]) // the overflow bucket, in list order
+        {
+            for (uint32_t q = tm.rank(); q < n_act; q += tm.size())
+                S.act[q] = S.color[S.alist[q]] == kColorSerial ? 1u : 0u;
+            tm.sync();
+            team_excl_scan(tm, S.act, S.act, n_act, S.tile_sums, sh);
+            for (uint32_t q = tm.rank(); q < n_act; q += tm.size())
+                if (S.color[S.alist[q]] == kColorSerial)
+                    S.loff[S.act[q]] = S.alist[q];
         }
         tm.sync();
         color_overflow(E, tm, W, S);
@@ -1322,11 +1332,11 @@ namespace rbps_gpu
             S.misc[kMiscCCount + x] = 0u;
         const uint32_t n_act = compact_grid(tm, S, n_cand, sh);
         if (n_act > kColorCtaMax)
-            color_rounds(E, tm, W, S, n_act);
+            color_rounds(E, tm, W, S, n_act, sh);
         else
         {
             if (blockIdx.x == 0)
-                color_rounds(E, BlockTeam(), W, S, n_act);
+                color_rounds(E, BlockTeam(), W, S, n_act, sh);
             tm.sync();
         }
         return S.misc[kMiscFlags + 1];
@@ -2693,7 +2703,8 @@ namespace rbps_gpu
 
     // Greedy colouring of the world's contacting candidates: in candidate
     // order, each takes the lowest colour free on both of its dynamic bodies
-    // (kColorSerial once a body has used all 64).  The team leader colours
+    // (kColorSerial once a body has used all 64; those are listed in S.loff
+    // in that order, which is the order they are relaxed in).  The team leader colours
     // sequentially with the per-body colour masks in `mask` (shared memory
     // when the world fits); the team then buckets the candidates by colour
     // (corder, colour offsets in misc).  The first substep of a step colours
@@ -2712,8 +2723,11 @@ namespace rbps_gpu
     // coloured in one round share no dynamic body, and the earliest
     // uncoloured one is always ready, so at most 32 rounds run.  claim holds
     // a word per body of scratch (the lowest uncoloured lane on the body).
+    // Those without a free colour go to `serial`, in list order but for ones
+    // of the same round.
     __device__ __forceinline__ void greedy_chunk_warp(const uint32_t *stage, uint8_t *scol, uint32_t m,
-                                                      unsigned long long *mask, uint32_t *cnt, uint32_t *claim)
+                                                      unsigned long long *mask, uint32_t *cnt, uint32_t *claim,
+                                                      const uint32_t *list, uint32_t *serial)
     {
         const uint32_t lane = threadIdx.x & 31u;
         for (uint32_t k0 = 0; k0 < m; k0 += 32)
@@ -2756,7 +2770,9 @@ namespace rbps_gpu
                             mask[b] |= bit;
                     }
                     scol[k] = (uint8_t)col;
-                    atomicAdd(&cnt[col], 1u);
+                    const uint32_t at = atomicAdd(&cnt[col], 1u);
+                    if (col == kColorSerial)
+                        serial[at] = list[k];
                     pending = false;
                 }
                 __syncwarp();
@@ -2832,7 +2848,7 @@ namespace rbps_gpu
                 if (claim)
                 {
                     if (tm.rank() < 32)
-                        greedy_chunk_warp(stage, scol, m, mask, cnt, claim);
+                        greedy_chunk_warp(stage, scol, m, mask, cnt, claim, S.alist + q0, S.loff);
                 }
                 else if (tm.leader())
                     for (uint32_t k = 0; k < m; ++k)
@@ -2852,6 +2868,8 @@ namespace rbps_gpu
                                 mask[b] |= bit;
                         }
                         scol[k] = (uint8_t)col;
+                        if (col == kColorSerial)
+                            S.loff[cnt[col]] = S.alist[q0 + k];
                         cnt[col] += 1u;
                     }
                 tm.sync();
@@ -2892,6 +2910,8 @@ namespace rbps_gpu
                                 mask[cd[k].bb] |= bit;
                         }
                         S.color[cs[k]] = col;
+                        if (col == kColorSerial)
+                            S.loff[cnt[col]] = cs[k];
                         cnt[col] += 1u;
                     }
             }
@@ -2949,6 +2969,18 @@ namespace rbps_gpu
             for (uint32_t k = tm.rank(); k < 66; k += tm.size())
                 misc[kMiscCOff + k] = off[k];
         tm.sync();
+        // the serial colour's slots in list order; the team's barrier after
+        // integrate comes before they are read (done in the fill above, the
+        // registers it took cost 4,096 worlds 1 % of a step)
+        if (book)
+            for (uint32_t q = off[kColorSerial] + tm.rank(); q < off[kColorSerial + 1]; q += tm.size())
+            {
+                const uint32_t c = S.loff[q - off[kColorSerial]];
+                if (in_smem)
+                    slots[q].x = c;
+                else
+                    S.corder[q] = c;
+            }
         if (!book) // the solves then take the overflow bucket by second-level colours
             color_overflow(E, tm, W, S);
         return book ? book[132] : misc[kMiscNColors];
