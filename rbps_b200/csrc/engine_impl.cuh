@@ -1159,13 +1159,17 @@ namespace rbps_gpu
                                  uint32_t n_act, BlockShared &sh)
     {
         uint32_t *misc = S.misc;
+        // uncoloured contacts per body, 32-bit words in bprio's space: what an
+        // earlier colouring left there would change how many colours a
+        // candidate draws from
+        uint32_t *ucnt = (uint32_t *)S.bprio;
         auto clear = [&](uint32_t b) {
             S.claim[(size_t)b * 64u + lane_id()] = 0ull;
             S.claim[(size_t)b * 64u + 32u + lane_id()] = 0ull;
             if (lane_id() == 0)
             {
                 S.bmask[b] = 0ull;
-                S.bprio[b] = 0ull;
+                ucnt[b] = 0u;
             }
         };
         const uint32_t warp = tm.rank() >> 5, warps = tm.size() >> 5;
@@ -1183,8 +1187,6 @@ namespace rbps_gpu
         const uint8_t *type = E.B.type + W.body_off;
         uint32_t round = 1;
         {
-            // uncoloured contacts per body (bprio's words reused as counters)
-            uint32_t *ucnt = (uint32_t *)S.bprio;
             for (uint32_t q = tm.rank(); q < n_act; q += tm.size())
             {
                 const Cand cd = S.cand[S.alist[q]];

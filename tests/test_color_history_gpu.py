@@ -13,8 +13,9 @@ pytestmark = pytest.mark.gpu
 FIELDS = ("position", "orientation", "linear_velocity", "angular_velocity")
 
 
-def scene(n, side=16):
-    """Ground, a plate with side^2 balls on it, and n balls in free fall."""
+def scene(n, gap, side=16):
+    """Ground, a plate with side^2 balls `gap` above it, a column of balls
+    that touch, and n balls in free fall."""
     rng = np.random.default_rng(1)
     bodies, forces, colliders = [], [], []
     scenes._ground(bodies, colliders, forces, 0.5, 0.0)
@@ -30,7 +31,10 @@ def scene(n, side=16):
     for k in range(side * side):
         x, z = 1.1 * (k % side - (side - 1) / 2), 1.1 * (k // side - (side - 1) / 2)
         r = float(rng.uniform(0.3, 0.4))
-        put((x, 0.39 + r - 0.01, z), abi.SHAPE_SPHERE, (r,), scenes.sphere_mass(r))
+        put((x, 0.39 + r + gap, z), abi.SHAPE_SPHERE, (r,), scenes.sphere_mass(r))
+    # their order shows in the state, and their bodies' words lie among the balls'
+    for k in range(12):
+        put((-20.0, 0.39 + 0.78 * k, 0.03 * (k % 3)), abi.SHAPE_SPHERE, (0.4,), scenes.sphere_mass(0.4))
     for k in range(n):
         put((3.0 * (k % 65) + 30.0, 50.0, 3.0 * (k // 65)), abi.SHAPE_SPHERE, (0.3,), scenes.sphere_mass(0.3))
     return scenes.Scene("plate", 1.0 / 60.0, 1, 0, [scenes._finish(bodies, forces, colliders, [])])
@@ -46,10 +50,32 @@ def test_runs_agree(rbps, n, precision):
     order within the serial colour is the list's."""
     states = []
     for _ in range(6):
-        b = rbps.Batch.from_scene(scene(n), precision, abi.SOLVE_COLORED)
+        b = rbps.Batch.from_scene(scene(n, -0.01), precision, abi.SOLVE_COLORED)
         b.step(1)
         assert b.stats()["serial_overflow"] > 128
         states.append(b.state_all(FIELDS))
     for st in states[1:]:
         for f in FIELDS:
             np.testing.assert_array_equal(st[f], states[0][f], err_msg=f)
+
+
+@pytest.mark.parametrize("precision", [abi.PRECISION_FP32, abi.PRECISION_FP64])
+@pytest.mark.parametrize("n", SIZES)
+def test_restored_run_repeats(rbps, n, precision):
+    """Whatever was coloured before: the colouring starts from cleared
+    counters, of the contacting bodies alone where they are few.  Here the
+    column's contacts are coloured before the balls land, and again after a
+    run in which they have."""
+    b = rbps.Batch.from_scene(scene(n, 0.02), precision, abi.SOLVE_COLORED)
+    slot = b.snapshot()
+    runs = []
+    for _ in range(3):
+        b.restore(slot)
+        b.step(1)
+        assert b.stats()["serial_overflow"] == 0 and b.stats()["contacts"] > 8
+        b.step(9)
+        assert b.stats()["serial_overflow"] > 0
+        runs.append(b.state_all(FIELDS))
+    for st in runs[1:]:
+        for f in FIELDS:
+            np.testing.assert_array_equal(st[f], runs[0][f], err_msg=f)
