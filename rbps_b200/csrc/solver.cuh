@@ -947,7 +947,8 @@ namespace rbps_gpu
                     rows[r].r2.w = cur.r2.w;
             }
         }
-        store_pose(B, i, X);
+        if (pl.b || j.b1 != j.b2) // a joint of a body with itself: body 2's copy is stored last
+            store_pose(B, i, X);
     }
 
     // Whether joint_damping does anything to the joint's bodies as they are.
