@@ -521,16 +521,67 @@ namespace rbps_gpu
     // overlap, so the pairs are exactly those of fat_overlap.  Most tests
     // fail on y or z: reading boxes by object through the endpoint list,
     // closing endpoints among them, once to count and once to emit, was most
-    // X  Hits go to S.pr_a / S.pr_b in
-    // no order, a warp's staging block at a time, and are then placed in the
-    // reference's emission order (by the later opening position, then the
-    // earlier one) by counting: a group's first slot plus the number of its
-    // entries with an earlier partner; groups past kGroupMax are radix
+    // of the frame (65,536 bodies 2.2 ms, 0.39 so).  Hits go to S.pr_a /
+    // S.pr_b in no order, a warp's staging block at a time, and are then
+    // placed in the reference's emission order (by the later opening position,
+    // then the earlier one) by counting: a group's first slot plus the number
+    // of its entries with an earlier partner; groups past kGroupMax are radix
     // sorted instead, which does not grow with their square.
     constexpr uint32_t kGroupMax = 64;
     constexpr uint32_t kSweepStage = 128; // hits a warp stages (words of BlockShared::wdig: 8 warps x 256)
 
+    // The pairs that a table of pair_cap too few keeps: the first by the
+    // earlier opening position, then the later, so that a world's state after
+    // a reported overflow is the same in every run.  Counts each object's
+    // pairs, scans, and emits up to the table's end; S.cnt as the sweep leaves
+    // it.  Only where more were found, after sweep_runs' own pass.
     template <class Team, class SC>
+    __device__ __noinline__ void sweep_kept(const Team &tm, const FatBox *fat, const uint32_t *ep_id, uint32_t n_open,
+                                            uint32_t pair_cap, const SC &S, BlockShared &sh, const float4 *yz)
+    {
+        const uint32_t *o_pos = S.ep_k2, *o_end = S.ep_v2;
+        const uint32_t lane = lane_id(), warps = tm.size() >> 5;
+        auto hits = [&](uint32_t k, uint32_t j) {
+            const bool hit = j < o_end[k] && yz_may_overlap(yz[k], yz[j]) &&
+                             fat_overlap(fat[ep_id[o_pos[k]] >> 1], fat[ep_id[o_pos[j]] >> 1]);
+            return __ballot_sync(0xffffffffu, hit);
+        };
+        for (uint32_t k = tm.rank() >> 5; k < n_open; k += warps)
+        {
+            uint32_t n = 0;
+            for (uint32_t j0 = k + 1; j0 < o_end[k]; j0 += 32)
+                n += __popc(hits(k, j0 + lane));
+            if (lane == 0)
+                S.cnt[k] = n;
+        }
+        tm.sync();
+        team_excl_scan(tm, S.cnt, S.cnt, n_open, S.tile_sums, sh);
+        for (uint32_t k = tm.rank() >> 5; k < n_open; k += warps)
+        {
+            uint32_t at = S.cnt[k];
+            for (uint32_t j0 = k + 1; j0 < o_end[k] && at < pair_cap; j0 += 32)
+            {
+                const uint32_t m = hits(k, j0 + lane), s = at + __popc(m & ((1u << lane) - 1u));
+                if ((m >> lane & 1u) && s < pair_cap)
+                {
+                    S.pr_a[s] = k;
+                    S.pr_b[s] = j0 + lane;
+                }
+                at += __popc(m);
+            }
+        }
+        tm.sync();
+        for (uint32_t k = tm.rank(); k <= n_open; k += tm.size())
+            S.cnt[k] = 0u;
+        tm.sync();
+        for (uint32_t s = tm.rank(); s < pair_cap; s += tm.size())
+            atomicAdd(&S.cnt[1u + S.pr_b[s]], 1u);
+        tm.sync();
+    }
+
+    // Keep: past pair_cap the pairs kept are the first ones (sweep_kept), not
+    // any, for callers that use them.
+    template <bool Keep, class Team, class SC>
     __device__ __noinline__ uint32_t sweep_runs(const Team &tm, const FatBox *fat, const uint32_t *ep_id,
                                                 const uint32_t *ep_pos, uint32_t nep, uint32_t id_limit,
                                                 uint32_t pair_cap, int *error, const SC &S, BlockShared &sh, float4 *yz)
@@ -632,6 +683,8 @@ namespace rbps_gpu
             if (tm.leader())
                 set_error(error, -2);
             total = pair_cap;
+            if constexpr (Keep)
+                sweep_kept(tm, fat, ep_id, n_open, pair_cap, S, sh, yz);
         }
         uint32_t largest = 0;
         for (uint32_t k = tm.rank(); k < n_open; k += tm.size())
@@ -707,8 +760,8 @@ namespace rbps_gpu
     // with the shared staging area sort_smem takes the fast paths above:
     // the merge of the endpoints flagged in `moved` (shared, one word per
     // endpoint position; null to sort in full) and the staged sweep.  yz:
-    // scratch, one per endpoint pair.
-    template <class Team, class SC>
+    // scratch, one per endpoint pair.  Keep: see sweep_runs.
+    template <bool Keep = false, class Team, class SC>
     __device__ __noinline__ uint32_t sap_sort_sweep(const Team &tm, const FatBox *fat, uint32_t *ep_key, uint32_t *ep_id,
                                        uint32_t *ep_pos, uint32_t nbp, uint32_t id_limit, uint32_t pair_cap,
                                        int *error, const SC &S, BlockShared &sh, float4 *yz,
@@ -767,7 +820,7 @@ namespace rbps_gpu
                     return total;
                 }
             }
-        const uint32_t total = sweep_runs(tm, fat, ep_id, ep_pos, nep, id_limit, pair_cap, error, S, sh, yz);
+        const uint32_t total = sweep_runs<Keep>(tm, fat, ep_id, ep_pos, nep, id_limit, pair_cap, error, S, sh, yz);
         sub_mark(prof, kPhSweep, tclk);
         for (uint32_t k = tm.rank(); k + 1 < total; k += tm.size())
             if (S.pk[k] > S.pk[k + 1])
@@ -841,8 +894,8 @@ namespace rbps_gpu
             }
         }
         tm.sync();
-        return sap_sort_sweep(tm, fat, ep_key, ep_id, ep_pos, nbp, nep, W.pair_cap, E.error, S, sh, S.yz, sort_smem,
-                              moved, prof);
+        return sap_sort_sweep<true>(tm, fat, ep_key, ep_id, ep_pos, nbp, nep, W.pair_cap, E.error, S, sh, S.yz,
+                                    sort_smem, moved, prof);
     }
 
     // Filtered SAP pairs followed by the plane candidates; returns the count.
