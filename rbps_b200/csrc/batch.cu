@@ -1928,10 +1928,11 @@ static int set_state_typed(rbps_batch *b, uint32_t first, uint32_t n, const rbps
     std::vector<V4<P>> pos(n);
     std::vector<Q4<T>> rot(n);
     std::vector<V4<T>> lin(n), ang(n);
-    CU(cudaMemcpy(pos.data(), (V4<P> *)b->pos + first, n * sizeof(V4<P>), cudaMemcpyDeviceToHost));
-    CU(cudaMemcpy(rot.data(), (Q4<T> *)b->rot + first, n * sizeof(Q4<T>), cudaMemcpyDeviceToHost));
-    CU(cudaMemcpy(lin.data(), (V4<T> *)b->lin + first, n * sizeof(V4<T>), cudaMemcpyDeviceToHost));
-    CU(cudaMemcpy(ang.data(), (V4<T> *)b->ang + first, n * sizeof(V4<T>), cudaMemcpyDeviceToHost));
+    CU(cudaMemcpyAsync(pos.data(), (V4<P> *)b->pos + first, n * sizeof(V4<P>), cudaMemcpyDeviceToHost, b->stream));
+    CU(cudaMemcpyAsync(rot.data(), (Q4<T> *)b->rot + first, n * sizeof(Q4<T>), cudaMemcpyDeviceToHost, b->stream));
+    CU(cudaMemcpyAsync(lin.data(), (V4<T> *)b->lin + first, n * sizeof(V4<T>), cudaMemcpyDeviceToHost, b->stream));
+    CU(cudaMemcpyAsync(ang.data(), (V4<T> *)b->ang + first, n * sizeof(V4<T>), cudaMemcpyDeviceToHost, b->stream));
+    CU(cudaStreamSynchronize(b->stream));
     for (uint32_t i = 0; i < n; ++i)
     {
         if (v->position)
@@ -1950,10 +1951,14 @@ static int set_state_typed(rbps_batch *b, uint32_t first, uint32_t n, const rbps
             ang[i] = V4<T>{T(v->angular_velocity[3 * i]), T(v->angular_velocity[3 * i + 1]),
                            T(v->angular_velocity[3 * i + 2]), T(0)};
     }
-    CU(cudaMemcpy((V4<P> *)b->pos + first, pos.data(), n * sizeof(V4<P>), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy((Q4<T> *)b->rot + first, rot.data(), n * sizeof(Q4<T>), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy((V4<T> *)b->lin + first, lin.data(), n * sizeof(V4<T>), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy((V4<T> *)b->ang + first, ang.data(), n * sizeof(V4<T>), cudaMemcpyHostToDevice));
+    // on the batch's stream, which waits for no other: a copy on the legacy
+    // stream may return before it has reached the device, and the next step
+    // or read would overtake it
+    CU(cudaMemcpyAsync((V4<P> *)b->pos + first, pos.data(), n * sizeof(V4<P>), cudaMemcpyHostToDevice, b->stream));
+    CU(cudaMemcpyAsync((Q4<T> *)b->rot + first, rot.data(), n * sizeof(Q4<T>), cudaMemcpyHostToDevice, b->stream));
+    CU(cudaMemcpyAsync((V4<T> *)b->lin + first, lin.data(), n * sizeof(V4<T>), cudaMemcpyHostToDevice, b->stream));
+    CU(cudaMemcpyAsync((V4<T> *)b->ang + first, ang.data(), n * sizeof(V4<T>), cudaMemcpyHostToDevice, b->stream));
+    CU(cudaStreamSynchronize(b->stream));
     return RBPS_OK;
 }
 
