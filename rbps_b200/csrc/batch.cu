@@ -487,12 +487,16 @@ struct rbps_batch
     size_t t_size() const { return desc.precision == RBPS_PRECISION_FP64 ? 8 : 4; }
     size_t p_size() const { return desc.precision == RBPS_PRECISION_FP64 ? 8 : 4; }
 
+    // Zeroed device memory, freed with the batch.  After the commit (which
+    // ends with a device synchronise) the fill runs on the batch's stream,
+    // where what is written next does: nothing orders that stream, which is
+    // non-blocking, behind a fill on the legacy one.
     int alloc(void **p, size_t bytes)
     {
         if (bytes == 0)
             bytes = 16;
         CU(cudaMalloc(p, bytes));
-        CU(cudaMemset(*p, 0, bytes));
+        CU(cudaMemsetAsync(*p, 0, bytes, committed ? stream : nullptr));
         allocs.push_back(*p);
         return RBPS_OK;
     }
@@ -1675,8 +1679,8 @@ static int alloc_dumps(rbps_batch *b)
     for (size_t w = 0; w < W; ++w)
         b->wdev[w].dump_slot = (uint32_t)w;
     CU(cudaMemcpy(b->worlds_d, b->wdev.data(), W * sizeof(WorldDev), cudaMemcpyHostToDevice));
-    // the zero fills above ran on the legacy stream; the step kernels run on
-    // the batch's non-blocking stream
+    // the copy above ran on the legacy stream; the step kernels run on the
+    // batch's non-blocking stream
     CU(cudaDeviceSynchronize());
     return RBPS_OK;
 }
@@ -2240,7 +2244,7 @@ static int debug_bp_typed(rbps_batch *b, uint32_t world, uint32_t *counts)
     Engine<T, P> e = make_engine<T, P>(b);
     uint32_t *d = nullptr;
     CU(cudaMalloc(&d, 16));
-    CU(cudaMemset(d, 0, 16));
+    CU(cudaMemsetAsync(d, 0, 16, b->stream));
     CU(launch_debug_broadphase<T, P>(e, world, b->block, d, b->stream));
     CU(cudaStreamSynchronize(b->stream));
     CU(cudaMemcpy(counts, d, 8, cudaMemcpyDeviceToHost));
@@ -2270,7 +2274,7 @@ extern "C" int rbps_batch_set_profile(rbps_batch *b, int32_t enable)
     if (enable && !b->prof && (rc = b->alloc((void **)&b->prof, bytes)))
         return rc;
     if (enable)
-        CU(cudaMemset(b->prof, 0, bytes));
+        CU(cudaMemsetAsync(b->prof, 0, bytes, b->stream));
     else
         b->prof_off = true;
     if (enable)
