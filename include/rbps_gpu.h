@@ -387,7 +387,11 @@ RBPS_API int rbps_batch_autotune(rbps_batch *batch, int32_t trial_steps, rbps_tu
  * depend on the configuration. */
 RBPS_API int rbps_batch_set_launch(rbps_batch *batch, const rbps_tune_result *config);
 
-/* Per-world body state, host doubles (converted from the device precision). */
+/* Per-world body state, host doubles (converted from the device precision).
+ * A batch's first read takes 1.7 MB of page-locked memory (about 2.5 ms where
+ * no ended batch has left its block); blocks of ended batches are kept for the
+ * next, no more than batches are alive and one at least.  A cudaDeviceReset
+ * frees them with the context; destroy the device's batches before it. */
 RBPS_API int rbps_batch_get_state(rbps_batch *batch, uint32_t world, const rbps_state_view *view);
 RBPS_API int rbps_batch_set_state(rbps_batch *batch, uint32_t world, const rbps_state_view *view);
 /* All worlds at once: bodies in world order (world 0 bodies, world 1 bodies, ...). */
@@ -475,7 +479,7 @@ RBPS_API int rbps_bp_configure(rbps_bp *bp, int32_t single_cta, int32_t block_th
  * synchronise the device; hosts that own a fixed device-memory budget).  The
  * SAP sort + sweep of n_objects fat AABBs as a freshly filled broadphase holds
  * them (endpoints in object order), with no allocation: working memory is a
- * file-scope device array of about 2.6 MB per GPU, held until exit.
+ * file-scope device array of about 2.4 MB per GPU, held until exit.
  *   fat_aabbs : device, 6 doubles per object {min.xyz, max.xyz}
  *   user_ids  : device, 1 per object
  *   pairs     : device, 2 * pair_cap; (id_a, id_b), id_a < id_b, in the

@@ -14,12 +14,14 @@
 #include <cstring>
 #include <limits>
 #include <memory>
-#include <mutex>
 #include <string>
 #include <vector>
 
+#include <cuda.h>
+
 #include "engine_types.cuh"
 #include "rbps_gpu.h"
+#include "staging.hpp"
 
 using namespace rbps_gpu;
 
@@ -321,60 +323,48 @@ struct HostHeightmap
 };
 
 // Page-locked staging of the state readback: two chunks of bodies and the
-// error words.  Locking its 1.7 MB takes a millisecond, more than a small
-// step, so a destroyed batch's goes to the next one: up to kKeep are kept,
-// the others unlocked.  A batch holds one from its first readback to its end
+// error words, 1.7 MB.  A batch holds one from its first readback to its end
 // and gives it back after its streams have drained.
 constexpr uint32_t kStateChunk = 8192; // bodies
+constexpr size_t kStateSlot = (size_t)kStateChunk * 13; // doubles
 
-struct StateStaging
+struct StagingApi
 {
-    static constexpr size_t kSlot = (size_t)kStateChunk * 13; // doubles
-    static constexpr size_t kKeep = 8;
-
-    static double *take()
+    // through the runtime: the library loads without a driver
+    template <class F>
+    static F driver(const char *name)
     {
-        {
-            std::lock_guard<std::mutex> lock(mutex());
-            if (!kept().empty())
-            {
-                double *p = kept().back();
-                kept().pop_back();
-                return p;
-            }
-        }
         void *p = nullptr;
-        return cudaHostAlloc(&p, (2 * kSlot + 8) * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped) ==
-                       cudaSuccess
-                   ? (double *)p
+        cudaDriverEntryPointQueryResult found;
+        return cudaGetDriverEntryPointByVersion(name, &p, 12000, cudaEnableDefault, &found) == cudaSuccess &&
+                       found == cudaDriverEntryPointSuccess
+                   ? (F)p
                    : nullptr;
     }
-    static void give(double *p)
+    static uint64_t context()
     {
-        {
-            std::lock_guard<std::mutex> lock(mutex());
-            if (kept().size() < kKeep)
-            {
-                kept().push_back(p);
-                return;
-            }
-        }
-        cudaFreeHost(p);
+        static const auto current = driver<CUresult (*)(CUcontext *)>("cuCtxGetCurrent");
+        static const auto id_of = driver<CUresult (*)(CUcontext, unsigned long long *)>("cuCtxGetId");
+        CUcontext c = nullptr;
+        unsigned long long id = 0;
+        if (current && id_of && current(&c) == CUDA_SUCCESS && c && id_of(c, &id) == CUDA_SUCCESS)
+            return id;
+        return 0;
     }
-
-private:
-    // never destroyed: a batch may outlive this file's statics
-    static std::mutex &mutex()
+    static void *lock(size_t bytes)
     {
-        static std::mutex &m = *new std::mutex;
-        return m;
+        void *p = nullptr;
+        return cudaHostAlloc(&p, bytes, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess ? p : nullptr;
     }
-    static std::vector<double *> &kept()
-    {
-        static std::vector<double *> &v = *new std::vector<double *>;
-        return v;
-    }
+    static void unlock(void *p) { cudaFreeHost(p); }
 };
+
+static StagingPool<StagingApi> &state_staging()
+{
+    // never destroyed: a batch may outlive this file's statics
+    static StagingPool<StagingApi> &pool = *new StagingPool<StagingApi>((2 * kStateSlot + 8) * sizeof(double));
+    return pool;
+}
 
 struct rbps_batch
 {
@@ -524,8 +514,8 @@ struct rbps_batch
     cudaEvent_t ev_force_ready[2] = {}, ev_force_free[2] = {}, ev_pose_ready[2] = {}, ev_out_free[2] = {};
     uint32_t io_slot = 0;
     bool io_async_ready = false;
-    // state readback (StateStaging)
-    double *state_host = nullptr;
+    // state readback (state_staging)
+    StagingBlock staging;
     cudaEvent_t ev_state[2] = {};
     // rbps_batch_collide's device buffer, kept up to kCollideKeep bytes
     static constexpr size_t kCollideKeep = size_t(64) << 20;
@@ -535,6 +525,7 @@ struct rbps_batch
     // the state arrays back to back
     std::vector<char *> snaps;
 
+    rbps_batch() { state_staging().begin(); }
     ~rbps_batch()
     {
         if (io_stream)
@@ -550,8 +541,12 @@ struct rbps_batch
         for (cudaEvent_t e : ev_state)
             if (e)
                 cudaEventDestroy(e);
-        if (state_host)
-            StateStaging::give(state_host);
+        int device = 0; // the caller's
+        cudaGetDevice(&device);
+        cudaSetDevice(desc.device);
+        staging.device = desc.device;
+        state_staging().end(staging);
+        cudaSetDevice(device);
         cudaFree(collide_dev);
         if (io_stream)
             cudaStreamDestroy(io_stream);
@@ -1889,18 +1884,19 @@ static int get_state_typed(rbps_batch *b, uint32_t first, uint32_t n, const rbps
             width += kWidth[f];
             mask |= 1u << f;
         }
-    if (!b->state_host && !(b->state_host = StateStaging::take()))
+    if (!b->staging.p && !(b->staging = state_staging().take(b->desc.device)).p)
         return fail(RBPS_ERR_CUDA, "rbps_batch_get_state: no page-locked memory");
+    double *const host = (double *)b->staging.p;
     for (cudaEvent_t &ev : b->ev_state)
         if (!ev)
             CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     const Engine<T, P> e = make_engine<T, P>(b);
     const uint32_t cap = kStateChunk, chunks = n && width ? (n + cap - 1) / cap : 0;
-    int *err = reinterpret_cast<int *>(b->state_host + 2 * StateStaging::kSlot);
+    int *err = reinterpret_cast<int *>(host + 2 * kStateSlot);
     auto issue = [&](uint32_t c) {
         const uint32_t i0 = c * cap, m = chunks ? std::min(cap, n - i0) : 0;
-        const cudaError_t rc = launch_state_out<T, P>(e, b->state_host + (c & 1) * StateStaging::kSlot, first + i0, m,
-                                                      mask, c ? nullptr : err, b->stream);
+        const cudaError_t rc = launch_state_out<T, P>(e, host + (c & 1) * kStateSlot, first + i0, m, mask,
+                                                      c ? nullptr : err, b->stream);
         return rc == cudaSuccess ? cudaEventRecord(b->ev_state[c & 1], b->stream) : rc;
     };
     CU(issue(0));
@@ -1915,7 +1911,7 @@ static int get_state_typed(rbps_batch *b, uint32_t first, uint32_t n, const rbps
             return check_device_error(b);
         }
         const uint32_t i0 = c * cap, m = std::min(cap, n - i0);
-        const double *from = b->state_host + (c & 1) * StateStaging::kSlot;
+        const double *from = host + (c & 1) * kStateSlot;
         for (int f = 0; f < 4 && chunks; ++f)
             if (to[f])
             {

@@ -60,7 +60,8 @@ namespace
     constexpr uint32_t oYz = (oErr + 4 + 3) / 4 * 4; // float4 per object
     constexpr uint32_t kScratchWords = oYz + 4 * kStaticMaxObjects;
 
-    // The working memory of rbps_sap_pairs_static (about 2.6 MB per GPU).
+    // The working memory of rbps_sap_pairs_static (about 2.4 MB per GPU).
+    static_assert(kScratchWords * 4ull > 2300000 && kScratchWords * 4ull < 2450000, "the figure stated here and in the header");
     static __device__ __align__(256) uint32_t g_sap_scratch[kScratchWords];
 
     struct StaticScr
