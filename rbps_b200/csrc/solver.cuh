@@ -929,6 +929,9 @@ namespace rbps_gpu
     {
         const PairLane pl;
         const uint32_t i = pl.b ? j.b2 : j.b1;
+        // a joint of a body with itself: body 2's copy is the one stored
+        const uint32_t partner = pl.other(i); // both lanes, not behind a short circuit
+        const bool stored = pl.b || partner != i;
         BodyR<T, P> X;
         load_body(B, i, X, false);
         if (j.type == kSpherical)
@@ -947,7 +950,7 @@ namespace rbps_gpu
                     rows[r].r2.w = cur.r2.w;
             }
         }
-        if (pl.b || j.b1 != j.b2) // a joint of a body with itself: body 2's copy is stored last
+        if (stored)
             store_pose(B, i, X);
     }
 
