@@ -985,14 +985,20 @@ namespace
     constexpr int kMaxBlockHost = 256; // block of the flat kernels (their __launch_bounds__)
     // The default team split: worlds of kBlockTeamBodies or more step on a
     // whole CTA, of kPairTeamBodies or more on half a CTA, others on a warp.
-    // Up to kFewWorldsPerSm worlds an SM every CTA is resident at once, and a
-    // smaller world has no one to leave the other warps to: CTAs from
-    // kPairTeamBodies on.  4,096 uneven worlds: 5.39 ms a step at 256 / 96,
-    // 5.18 at 192 / 64; 256 towers of 65 bodies: 1.68 ms on warps, 1.53 on
-    // CTAs; 61 uneven worlds: 0.82 either way.
+    // Where a CTA for each world would be resident at once, a smaller world
+    // has no one to leave the other warps to: CTAs from kPairTeamBodies on.
+    // 4,096 uneven worlds: 5.39 ms a step at 256 / 96, 5.18 at 192 / 64; 256
+    // towers of 65 bodies: 1.68 ms on warps, 1.53 on CTAs; 61 uneven worlds:
+    // 0.82 either way.  How many are resident is asked of the kernel, with the
+    // shared memory of that split: up to three an SM in float, two in double,
+    // fewer with large worlds (double, 64 to 256 bodies: 296 worlds 0.90 ms a
+    // step on CTAs and 0.92 at 192 / 64, 330 worlds 1.13 and 0.96, 444 worlds
+    // 1.38 and 1.08; 200 worlds of 64 to 900 bodies 1.80 and 1.59.  Float, 444
+    // worlds: 64 to 256 bodies 0.59 and 0.63, but 8 to 128 bodies 0.59 and
+    // 0.55, where the worlds on warps are the last to end).
     constexpr uint32_t kBlockTeamBodies = 192;
     constexpr uint32_t kPairTeamBodies = 64;
-    constexpr uint32_t kFewWorldsPerSm = 3;
+    constexpr uint32_t kFewWorldsPerSm = 3; // no kernel has more CTAs resident in that split
     constexpr size_t kSmemWorldsMax = 226 * 1024; // bytes of world copies a CTA can open (227 KB less the scan words)
     constexpr uint32_t kSmemBodiesMax = 1024;   // bodies a CTA world keeps in shared memory (137 KB in FP32)
 } // namespace
@@ -1587,8 +1593,15 @@ static int commit_typed(rbps_batch *b)
         b->flat.grid_sort = std::max(1, per_sm) * b->sm_count;
         b->flat.block_solve = 128;
         b->flat.sm_count = b->sm_count;
-        const bool few = ns <= kFewWorldsPerSm * (uint32_t)b->sm_count;
-        if ((rc = set_team_split<T, P>(b, few ? kPairTeamBodies : kBlockTeamBodies, kPairTeamBodies)))
+        bool few = ns <= kFewWorldsPerSm * (uint32_t)b->sm_count;
+        if (few)
+        {
+            if ((rc = set_team_split<T, P>(b, kPairTeamBodies, kPairTeamBodies)))
+                return rc;
+            CU(occupancy_flat<T, P>(1, b->flat.block_solve, &per_sm, b->flat.substep_smem));
+            few = ns <= (uint32_t)(per_sm * b->sm_count);
+        }
+        if (!few && (rc = set_team_split<T, P>(b, kBlockTeamBodies, kPairTeamBodies)))
             return rc;
     }
     for (const auto &w : b->worlds)

@@ -3416,7 +3416,7 @@ namespace rbps_gpu
         return cudaGetLastError();
     }
 
-    // kernel 0: narrowphase, 1: substep, 2: class sort
+    // kernel 0: narrowphase, 1: substep (the variant of launches that fit), 2: class sort
     template <class T, class P>
     cudaError_t occupancy_flat(int kernel, int block, int *blocks_per_sm, size_t fl_smem)
     {
@@ -3431,7 +3431,8 @@ namespace rbps_gpu
             *blocks_per_sm = a < b ? a : b;
             return rc;
         }
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_substep<T, P, false, kSubstepBlocks<T>>, block, fl_smem);
+        constexpr int kFits = sizeof(T) == 8 ? kSubstepBlocks<T> : kSubstepBlocksFew;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_substep<T, P, false, kFits>, block, fl_smem);
     }
 
     // Enqueues one step of one large world: one cooperative launch, or with a
