@@ -1527,12 +1527,13 @@ static int commit_typed(rbps_batch *b)
     }
     const size_t ccs = cc_size_of(b->desc.precision);
     // per-world scratch slices
+    const bool levels = b->desc.solve_mode == RBPS_SOLVE_REFERENCE_ORDER;
     size_t scr_total = 0;
     for (uint32_t w = 0; w < W; ++w)
     {
         WorldDev &d = b->wdev[w];
         d.scr_off = scr_total;
-        scr_total += make_layout(d.n_bp, d.n_bodies, d.pair_cap, d.n_pc, ccs).stride;
+        scr_total += make_layout(d.n_bp, d.n_bodies, d.pair_cap, d.n_pc, ccs, levels).stride;
     }
     if ((rc = b->alloc((void **)&b->scratch, std::max<size_t>(scr_total, 256))))
         return rc;
@@ -1776,7 +1777,8 @@ template <class T, class P>
 static int step_typed(rbps_batch *b, int n)
 {
     // side stream + events for the parallel narrowphase kernels, with the
-    // first step: a batch that only answers queries has no use for them
+    // first step (50 us of 1.7 ms, most of it the graph's capture): a batch
+    // that only answers queries has no use for them
     if (!b->small_ids.empty() && n > 0 && !b->flat.side)
     {
         for (cudaEvent_t *ev : {&b->flat.fork, &b->flat.join})

@@ -70,7 +70,8 @@ namespace rbps_gpu
         size_t corder;           // candidates sorted by colour
         size_t misc;             // small counters
         size_t act, alist;       // active-candidate flags (then levels) / compacted list
-        size_t lrec, loff;       // reference order: packed bodies of the active candidates, level offsets
+        size_t loff;             // reference order: level offsets; else the serial colour's candidates
+        size_t lrec;             // reference order: packed bodies of the active candidates
         size_t stride;           // bytes per executor
     };
 
@@ -112,7 +113,10 @@ namespace rbps_gpu
     constexpr uint32_t kMiscColorValid = kMiscC2Off + 66;
     static_assert(kMiscColorValid < kMiscWords, "misc words");
 
-    RBPS_HD ScratchLayout make_layout(uint32_t nbp, uint32_t nb, uint32_t pair_cap, uint32_t npc, size_t cc_size)
+    // levels: the batch steps in reference order (the device takes it so: it
+    // has no use for the stride)
+    RBPS_HD ScratchLayout make_layout(uint32_t nbp, uint32_t nb, uint32_t pair_cap, uint32_t npc, size_t cc_size,
+                                      bool levels = true)
     {
         ScratchLayout L{};
         const size_t nep = 2 * (size_t)nbp + 1;
@@ -154,8 +158,9 @@ namespace rbps_gpu
         take(L.misc, kMiscWords * 4);
         take(L.act, nc * 4);
         take(L.alist, nc * 4);
-        take(L.lrec, nc * 8);
         take(L.loff, (nc + 1) * 4);
+        if (levels) // last: the other offsets are the same in both modes
+            take(L.lrec, nc * 8);
         L.stride = scr_align(off, 256);
         return L;
     }
@@ -304,7 +309,7 @@ namespace rbps_gpu
         size_t substep_smem; // dynamic shared memory of k_substep
         bool triangles, others; // the batch has meshes or heightmaps / other kinds beyond sphere, box, capsule, plane
         // a second stream on which the box-box narrowphase runs beside the
-        // other classes' (fork / join events), or null for one stream
+        // other classes' (fork / join events)
         cudaStream_t side;
         cudaEvent_t fork, join;
     };
