@@ -41,7 +41,8 @@ extern "C" {
 enum {
     RBPS_OK = 0,
     RBPS_ERR_INVALID = -1,       /* bad argument / call order              */
-    RBPS_ERR_CAPACITY = -2,      /* a device buffer (pairs, contacts, ...) overflowed */
+    RBPS_ERR_CAPACITY = -2,      /* a device buffer (pairs, contacts, ...) overflowed; a step keeps the first
+                                  * max_pairs_per_world pairs by the earlier object's place in the sweep */
     RBPS_ERR_CUDA = -3,          /* CUDA runtime failure                   */
     RBPS_ERR_NOT_CONVERGED = -4, /* an iterative kernel hit its iteration cap */
     RBPS_ERR_STATE = -5,         /* non-finite body state detected          */

@@ -9,11 +9,12 @@
 
 namespace rbps_gpu
 {
-    // Warps per CTA of the GJK kernels; each warp owns gjk_warp_bytes (21 KB)
+    // Warps per CTA of the GJK kernels; each warp owns gjk_warp_bytes (27 KB)
     // of the CTA's dynamic shared memory.  Eight warps an SM leave a thread
     // 255 registers, which hold the simplex and both shapes' transforms.
     constexpr int kGjkWarps = 4;
     constexpr size_t kGjkWarpBytes = gjk_warp_bytes<double>();
+    static_assert(kGjkWarpBytes > 27000 && kGjkWarpBytes < 28000, "the figure above");
     constexpr size_t kGjkSmem = kGjkWarps * kGjkWarpBytes;
 
     // Opens a GJK kernel to its shared workspaces (once per device and kernel).
