@@ -1578,6 +1578,47 @@ namespace rbps_gpu
         store_vel(B, bb, Bb);
     }
 
+    // The rows of the overflow bucket (contacts past a body's 64 colours).  In
+    // float the compiler chooses for each inlined copy of a row which products
+    // contract, so with a copy in every team's code a world's last bits hung
+    // on the launch shape: k_substep calls one copy (Out).  The kernels that
+    // keep one team keep their inlined copies, and their bits.  Out of line
+    // they also leave the four-CTA float kernel 580 bytes of spills instead of
+    // 880 (4,096 worlds, four steps: 21.80 ms before, 21.57 so).
+    template <class T, class P>
+    __device__ __noinline__ void solve_position_call(const Bodies<T, P> &B, T inv_h, uint32_t ba, uint32_t bb,
+                                                     CandContacts<T, P> &cc)
+    {
+        solve_pair_position(B, inv_h, ba, bb, cc);
+    }
+
+    template <class T, class P>
+    __device__ __noinline__ void solve_velocity_call(const Bodies<T, P> &B, T h, uint32_t ba, uint32_t bb,
+                                                     const CandContacts<T, P> &cc)
+    {
+        solve_pair_velocity(B, h, ba, bb, cc);
+    }
+
+    template <bool Out, class T, class P>
+    __device__ __forceinline__ void solve_overflow_position(const Bodies<T, P> &B, T inv_h, uint32_t ba, uint32_t bb,
+                                                            CandContacts<T, P> &cc)
+    {
+        if constexpr (Out)
+            solve_position_call(B, inv_h, ba, bb, cc);
+        else
+            solve_pair_position(B, inv_h, ba, bb, cc);
+    }
+
+    template <bool Out, class T, class P>
+    __device__ __forceinline__ void solve_overflow_velocity(const Bodies<T, P> &B, T h, uint32_t ba, uint32_t bb,
+                                                            const CandContacts<T, P> &cc)
+    {
+        if constexpr (Out)
+            solve_velocity_call(B, h, ba, bb, cc);
+        else
+            solve_pair_velocity(B, h, ba, bb, cc);
+    }
+
     // The same with a pair of lanes, a body each (solver.cuh).
     template <class T, class P>
     __device__ __forceinline__ void solve_pair_position_split(const Bodies<T, P> &B, uint32_t ba, uint32_t bb,
@@ -1896,8 +1937,8 @@ namespace rbps_gpu
     }
 
     // Ref: the reference's order, level by level (schedule_levels), else
-    // colour by colour.
-    template <bool Ref, class T, class P, class Team>
+    // colour by colour.  Out: see solve_position_call.
+    template <bool Ref, bool Out = false, class T, class P, class Team>
     __device__ void phase_position_on(const Engine<T, P> &E, const Team &tm, uint32_t w, const Bodies<T, P> &B,
                                       uint32_t boff, const uint32_t *book = nullptr, const uint2 *slots = nullptr)
     {
@@ -1951,7 +1992,7 @@ namespace rbps_gpu
                     sweep_colors(tm, c2, kColorSerial, [&](uint32_t q) {
                         const uint32_t c = S.corder[q];
                         const Cand cd = S.cand[c];
-                        solve_pair_position(B, E.inv_h, boff + cd.ba, boff + cd.bb, S.cc[c]);
+                        solve_overflow_position<Out>(B, E.inv_h, boff + cd.ba, boff + cd.bb, S.cc[c]);
                     });
                     serial0 = c2[kColorSerial];
                 }
@@ -1960,7 +2001,7 @@ namespace rbps_gpu
                     {
                         const uint32_t c = sl ? slots[q].x : S.corder[q];
                         const Cand cd = S.cand[c];
-                        solve_pair_position(B, E.inv_h, boff + cd.ba, boff + cd.bb, S.cc[c]);
+                        solve_overflow_position<Out>(B, E.inv_h, boff + cd.ba, boff + cd.bb, S.cc[c]);
                     }
                 tm.sync();
             }
@@ -2011,7 +2052,7 @@ namespace rbps_gpu
     }
 
     // Velocity solve (World.hpp:176-180): restitution / friction, joint damping.
-    template <bool Ref, class T, class P, class Team>
+    template <bool Ref, bool Out = false, class T, class P, class Team>
     __device__ void phase_velocity_on(const Engine<T, P> &E, const Team &tm, uint32_t w, const Bodies<T, P> &B,
                                       uint32_t boff, const uint32_t *book = nullptr, const uint2 *slots = nullptr)
     {
@@ -2063,7 +2104,7 @@ namespace rbps_gpu
                     sweep_colors(tm, c2, kColorSerial, [&](uint32_t q) {
                         const uint32_t c = S.corder[q];
                         const Cand cd = S.cand[c];
-                        solve_pair_velocity(B, E.h, boff + cd.ba, boff + cd.bb, S.cc[c]);
+                        solve_overflow_velocity<Out>(B, E.h, boff + cd.ba, boff + cd.bb, S.cc[c]);
                     });
                     serial0 = c2[kColorSerial];
                 }
@@ -2072,7 +2113,7 @@ namespace rbps_gpu
                     {
                         const uint32_t c = sl ? slots[q].x : S.corder[q];
                         const Cand cd = S.cand[c];
-                        solve_pair_velocity(B, E.h, boff + cd.ba, boff + cd.bb, S.cc[c]);
+                        solve_overflow_velocity<Out>(B, E.h, boff + cd.ba, boff + cd.bb, S.cc[c]);
                     }
                 tm.sync();
             }
@@ -3214,8 +3255,8 @@ namespace rbps_gpu
                 integrate_body(V, boff + b, E.h);
         tm.sync();
         clk.mark(kPhIntegrate);
-        phase_position_on<Ref>(E, tm, w, V, boff, book, slots);
-        phase_velocity_on<Ref>(E, tm, w, V, boff, book, slots);
+        phase_position_on<Ref, true>(E, tm, w, V, boff, book, slots);
+        phase_velocity_on<Ref, true>(E, tm, w, V, boff, book, slots);
         if (local)
         {
             const Bodies<T, P> &G = E.B;

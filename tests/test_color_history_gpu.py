@@ -79,3 +79,19 @@ def test_restored_run_repeats(rbps, n, precision):
     for st in runs[1:]:
         for f in FIELDS:
             np.testing.assert_array_equal(st[f], runs[0][f], err_msg=f)
+
+
+@pytest.mark.parametrize("precision", [abi.PRECISION_FP32, abi.PRECISION_FP64])
+def test_launch_shapes_agree(rbps, precision):
+    """A CTA, half a CTA and a warp relax the serial colour in one order."""
+    states = []
+    for team, pair in ((1, 1), (5000, 2), (5000, 5000)):
+        b = rbps.Batch.from_scene(scene(0, -0.01), precision, abi.SOLVE_COLORED)
+        b.set_launch(team_bodies=team, pair_bodies=pair)
+        b.step(1)
+        assert b.stats()["serial_overflow"] > 128
+        b.step(3)
+        states.append(b.state_all(FIELDS))
+    for st in states[1:]:
+        for f in FIELDS:
+            np.testing.assert_array_equal(st[f], states[0][f], err_msg=f)
