@@ -3096,7 +3096,7 @@ namespace rbps_gpu
     // In double a pair's two bodies alone take 104 registers: two CTAs (255).
     template <class T> constexpr int kSubstepBlocks = sizeof(T) == 8 ? 2 : RBPS_SUBSTEP_MIN_BLOCKS;
     // A launch whose CTAs are all resident at three an SM gains nothing from
-    // a fourth slot, and at 168 registers a float row spills nothing: 61
+    // a fourth slot, and at 168 registers a thread spills 56 bytes, not 580: 61
     // worlds of up to 512 bodies, two steps, 2.10 ms at 128 registers and
     // 1.99 at 168; 256 towers of 64 boxes 2.51 and 2.26 (two CTAs, 255
     // registers: 1.99 and 2.25).
